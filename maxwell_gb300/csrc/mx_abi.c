@@ -342,16 +342,23 @@ int addeval_edge2d_gpu(mxg_field alpha, mxg_field beta, const edge2d_gpu *x, edg
 int addeval_shifted_edge2d_gpu(double alpha, const double *beta, const edge2d_gpu *x, edge2d_gpu *y)
 {
   const grid2d_gpu *g = x->gr;
-  size_t km = (size_t) g->K * x->m;
-  double *d;
+  size_t km = (size_t) g->K * x->m, i;
+  mxk_scalar *h, *d;
   int e;
   if(!same_shape_e(x, y)) return MXG_EINVAL;
-  if(cudaMalloc((void **) &d, sizeof(double) * km)) return MXG_ENOMEM;
-  e = (int) cudaMemcpy(d, beta, sizeof(double) * km, cudaMemcpyHostToDevice);
+  h = malloc(sizeof(mxk_scalar) * km);
+  if(!h || cudaMalloc((void **) &d, sizeof(mxk_scalar) * km)) { free(h); return MXG_ENOMEM; }
+  for(i = 0; i < km; i++) {
+    h[i].d = beta[i] / 6.0;
+    h[i].hi = (float) h[i].d;
+    h[i].lo = (float) (h[i].d - (double) h[i].hi);
+  }
+  e = (int) cudaMemcpy(d, h, sizeof(mxk_scalar) * km, cudaMemcpyHostToDevice);
   if(!e) e = mxk_edge_apply(g->n, x->m, g->K, g->ph, kap_of(g), alpha, 0.0, d, 1.0, x->prec, x->d, y->prec, 0, y->d,
                             g->st);
   if(!e) e = (int) cudaStreamSynchronize(g->st);
   cudaFree(d);
+  free(h);
   return e;
 }
 

@@ -128,6 +128,12 @@ template <typename R> __device__ __forceinline__ cx<R> czero() { return mkc(Real
 template <typename R> __device__ __forceinline__ cx<R> cfrom(double re, double im) {
   return mkc(Real<R>::from(re), Real<R>::from(im));
 }
+// 4 a, exact in every arithmetic (for a float-float number two products
+// instead of a full multiplication)
+__device__ __forceinline__ float times4(float a) { return 4.0f * a; }
+__device__ __forceinline__ double times4(double a) { return 4.0 * a; }
+__device__ __forceinline__ dd times4(dd a) { return dd_make(4.0f * a.hi, 4.0f * a.lo); }
+template <typename R> __device__ __forceinline__ cx<R> times4(cx<R> a) { return mkc(times4(a.re), times4(a.im)); }
 // exactly representable literal constants (no double arithmetic at run time)
 template <typename R> __device__ __forceinline__ R rc(float f) { return Real<R>::from_float(f); }
 
@@ -135,7 +141,8 @@ template <typename R> __device__ __forceinline__ R rc(float f) { return Real<R>:
 // Scalars prepared on the host in all three arithmetics.  GB300 issues FP64
 // instructions at a small fraction of its FP32 rate, so the FP32 and
 // float-float kernels never compute or convert a constant in double: every
-// run-time scalar arrives as (double, float hi, float lo).
+// run-time scalar arrives as (double, float hi, float lo); arrays of them
+// have the layout of mxk_scalar (mx_internal.h).
 // ------------------------------------------------------------------
 struct Sc {
   double d;

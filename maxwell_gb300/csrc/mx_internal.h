@@ -50,10 +50,17 @@ typedef struct {
 int mxk_afw_factors(int n, const float *kappa_f, double alpha, double beta, void *out, mx_stream s);
 
 /* ---- edge space ---- */
-/* y = cy*(yin ? yin : y) + alpha*A x + beta_kv*M x; beta_kv (K*m doubles)
- * or NULL -> beta; yin (precision prec_y) may be NULL; cy = 0 reads neither */
+/* a real scalar in double and as a float-float pair (device arrays of
+ * per-vector scalars, so that no kernel converts one in double arithmetic) */
+typedef struct {
+  double d;
+  float hi, lo;
+} mxk_scalar;
+/* y = cy*(yin ? yin : y) + alpha*A x + beta*M x, with a beta of its own per
+ * (k, vector) where mm_kv (K*m device scalars beta / 6) is not NULL; yin
+ * (precision prec_y) may be NULL; cy = 0 reads neither */
 int mxk_edge_apply(int n, int m, int K, const double *phases, mxk_kappa kap,
-                   double alpha, double beta, const double *beta_kv, double cy,
+                   double alpha, double beta, const mxk_scalar *mm_kv, double cy,
                    int prec_x, const void *x, int prec_y, const void *yin, void *y, mx_stream s);
 /* AFW line Gauss-Seidel sweep in the reference's row order; dir 0 forward,
  * 1 backward, 2 symmetric (forward then backward) */

@@ -151,41 +151,91 @@ __device__ __forceinline__ cx<R> mx_y(const A& E, R mm, int i, int j) {
 // edge operator
 // ------------------------------------------------------------------
 // y = cy * (yin ? yin : y) + axy*A x + mm*M x; axy = alpha n^2, mm = beta/6
-// (per (k, v) from beta_kv when given: that form converts in double and
-// serves the shifted operator of the mirror API only)
+// (per (k, v) from mm_kv when given, in all three arithmetics: dividing and
+// converting a double shift per thread was bound by the FP64 rate)
+//
+// A CTA marches up a strip of EA_ROWS (or fewer) rows; a thread owns a cell
+// column and a vector.  It forms the row's curl times kappa once; the cell
+// below is its own of the row before, and the x-edges of rows j-1 and j stay
+// in registers.  The cell to the left: c64 blocks are bound by memory, a
+// thread forms it a second time from two more loads and nothing waits;
+// float-float and FP64 blocks are bound by arithmetic (a float-float add is
+// 20 FP32 instructions), the neighbour thread hands it over through shared
+// memory and the first column of a tile only supplies it.
+// Measured against a thread per (site, vector), 512^2 cells x 16 vectors:
+// shifted defect, cdd into c64, 8 k-points 1.46 -> 1.03 ms (issue slots 76 %
+// busy; three CTAs per SM, 1.17 ms with two); c64 residual, 32 k-points
+// 1.59 -> 1.46 ms (4.4 TB/s), 64^2 x 12 x 8 k-points 12.6 -> 10.6 us.
+constexpr int EA_ROWS = 8;
+template <typename R> struct EaShare { static constexpr bool value = sizeof(R) > 4; };
 template <typename SX, typename SY, typename R>
-__global__ void k_edge_apply(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap, Sc axy_s,
-                             Sc mm_s, const double* __restrict__ beta_kv, Sc cy_s, int has_cy,
-                             const SX* __restrict__ x, const SY* yin, SY* y) {
-  // block (m, rows): x = vector, y = site; grid.y = k-point
-  int k = blockIdx.y, v = threadIdx.x;
-  int site = blockIdx.x * blockDim.y + threadIdx.y;
-  if (site >= n * n) return;
-  int i = site % n, j = site / n;
+__global__ void __launch_bounds__(256, 3) k_edge_apply(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap,
+                                                    Sc axy_s, Sc mm_s, const Sc* __restrict__ mm_kv, Sc cy_s,
+                                                    int has_cy, int rj, const SX* __restrict__ x, const SY* yin,
+                                                    SY* y) {
+  // block (m, columns): x = vector, y = cell column; grid (column tiles, strips, K)
+  constexpr bool SH = EaShare<R>::value;
+  __shared__ cx<R> left[2][SH ? 256 : 1];
+  const int k = blockIdx.z, v = threadIdx.x, ty = threadIdx.y, at = ty * blockDim.x + v;
+  const int i = SH ? (int) (blockIdx.x * (blockDim.y - 1) + ty) - 1 : (int) (blockIdx.x * blockDim.y + ty);
+  const int j0 = blockIdx.y * rj, j1 = j0 + rj < n ? j0 + rj : n;
+  const bool cell = i < n;
+  if (!SH && !cell) return;
   Lay L{n, m, K};
-  R axy = sget<R>(axy_s);
-  R mm = beta_kv ? Real<R>::from(beta_kv[(size_t) k * m + v] / 6.0) : sget<R>(mm_s);
+  const R axy = sget<R>(axy_s);
+  const R mm = sget<R>(mm_kv ? mm_kv[(size_t) k * m + v] : mm_s);
   const SX* xb = x + L.edge(k, 0, 0, 0, v);
-  cx<R> ox, oy;
-  if (i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-    EAccI<SX, R> E{xb, n, m};
-    KapI<R> ki{kap};
-    ox = kx_x<R>(E, ki, axy, mm, i, j);
-    oy = kx_y<R>(E, ki, axy, mm, i, j);
-  } else {
-    EAcc<SX, R> E{xb, n, m, seam_load<R>(ph, K, k, n)};
-    ox = kx_x<R>(E, kap, axy, mm, i, j);
-    oy = kx_y<R>(E, kap, axy, mm, i, j);
+  const bool icol = i > 0 && i < n - 1;
+  // x(i, j-1..j+1), y(i-1..i+1, j), kappa curl of cells (i, j), (i, j-1), (i-1, j)
+  cx<R> xm, x0, xp, yl, y0, yr, kc, kb, kl, w0, wp;
+  auto row = [&](const auto& E, const auto& KA, int j, bool halo) {
+    xp = E(0, i, j + 1);
+    y0 = E(1, i, j);
+    yr = E(1, i + 1, j);
+    kc = scal(KA(i, j), x0 - xp - y0 + yr);
+    if (!SH) wp = E(0, i - 1, j + 1);
+    if (halo) return;
+    yl = E(1, i - 1, j);
+    if (!SH) kl = scal(KA(i - 1, j), w0 - wp - yl + y0);
+  };
+  EAccI<SX, R> EI{xb, n, m};
+  EAcc<SX, R> ES{xb, n, m, seam_load<R>(ph, K, k, n)};
+  const KapI<R> KI{kap};
+  if (cell) {
+    // the row below the strip: its x-edges and cell
+    const bool in = icol && j0 > 0;
+    x0 = in ? EI(0, i, j0 - 1) : ES(0, i, j0 - 1);
+    if (in) row(EI, KI, j0 - 1, true);
+    else row(ES, kap, j0 - 1, true);
   }
-  size_t ox_at = L.edge(k, 0, j, i, v), oy_at = L.edge(k, 1, j, i, v);
-  if (has_cy) {
-    const SY* src = yin ? yin : y;
-    R c = sget<R>(cy_s);
-    ox += scal(c, Store<SY, R>::ld(src + ox_at));
-    oy += scal(c, Store<SY, R>::ld(src + oy_at));
+  for (int j = j0, q = 0; j < j1; j++, q ^= 1) {
+    if (cell) {
+      xm = x0;
+      x0 = xp;
+      kb = kc;
+      if (!SH) w0 = wp;
+      if (icol && j < n - 1) row(EI, KI, j, false);
+      else row(ES, kap, j, false);
+    }
+    if (SH) {
+      left[q][at] = kc;
+      __syncthreads();   // (row j + 2 reuses the buffer, past the barrier of row j + 1)
+      if (!cell || ty == 0) continue;
+      kl = left[q][at - blockDim.x];
+    }
+    cx<R> ox = scal(axy, kc - kb) + scal(mm, times4(x0) + xp + xm);
+    cx<R> oy = scal(axy, kl - kc) + scal(mm, times4(y0) + yr + yl);
+    const size_t ox_at = L.edge(k, 0, j, i, v), oy_at = L.edge(k, 1, j, i, v);
+    if (has_cy) {
+      const SY* src = yin ? yin : y;
+      const cx<R> sx = Store<SY, R>::ld(src + ox_at), sy = Store<SY, R>::ld(src + oy_at);
+      const R c = sget<R>(cy_s);
+      ox += has_cy == 1 ? sx : scal(c, sx);   // has_cy 1: cy is 1
+      oy += has_cy == 1 ? sy : scal(c, sy);
+    }
+    Store<SY, R>::st(y + ox_at, ox);
+    Store<SY, R>::st(y + oy_at, oy);
   }
-  Store<SY, R>::st(y + ox_at, ox);
-  Store<SY, R>::st(y + oy_at, oy);
 }
 
 // ------------------------------------------------------------------
@@ -1529,14 +1579,19 @@ extern "C" int mxk_afw_factors(int n, const float* kappa_f, double alpha, double
 }
 
 extern "C" int mxk_edge_apply(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,
-                              double beta, const double* beta_kv, double cy, int px, const void* x,
+                              double beta, const mxk_scalar* mm_kv, double cy, int px, const void* x,
                               int py, const void* yin, void* y, mx_stream s) {
-  dim3 g = grd2((size_t) n * n, m, K), b = blk2(m);
+  const dim3 b = blk2(m);
   cudaStream_t st = (cudaStream_t) s;
   Sc axy = make_sc(alpha * (double) n * (double) n), mm = make_sc(beta / 6.0), c = make_sc(cy);
-  int has = cy != 0.0;
+  int has = cy == 0.0 ? 0 : cy == 1.0 ? 1 : 2;
+  // strips of EA_ROWS rows where that leaves at least two full loads of
+  // threads for the GPU, shorter ones (down to a row) below
+  const size_t fill = (size_t) n * n * m * K / ((size_t) 2 * 2048 * 152);
+  const int rj = fill >= EA_ROWS ? EA_ROWS : fill > 1 ? (int) fill : 1;
+  const dim3 g1((n + b.y - 1) / b.y, (n + rj - 1) / rj, K), g2((n + b.y - 2) / (b.y - 1), (n + rj - 1) / rj, K);
 #define MX_EA(SX, SY, R)                                                                              \
-  k_edge_apply<SX, SY, R><<<g, b, 0, st>>>(n, m, K, ph, make_kap<R>(kap, n), axy, mm, beta_kv, c, has, \
+  k_edge_apply<SX, SY, R><<<EaShare<R>::value ? g2 : g1, b, 0, st>>>(n, m, K, ph, make_kap<R>(kap, n), axy, mm, (const Sc*) mm_kv, c, has, rj, \
                                            (const SX*) x, (const SY*) yin, (SY*) y)
   if (px == MX_C64 && py == MX_C64) MX_EA(float2, float2, float);
   else if (px == MX_C128 && py == MX_C128) MX_EA(double2, double2, double);

@@ -1,0 +1,37 @@
+"""Kernels whose launch shape depends on the size, at the sizes where the
+shape changes, against the oracle.  Tolerances are those of the operators'
+own tests (the storage's arithmetic)."""
+import numpy as np
+import pytest
+
+import maxwell_gb300 as mx
+
+pytestmark = pytest.mark.gpu
+
+TOL = {mx.C128: 1e-12, mx.CDD: 1e-12, mx.C64: 2e-5}
+FACTORS = np.array([[np.exp(0.7j), np.exp(-1.3j)], [1.0, 1.0], [np.exp(2.9j), np.exp(0.4j)]])
+
+
+def rel(a, b):
+    return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
+
+
+def cv(rng, *shape):
+    return rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+
+
+@pytest.mark.parametrize("n, m, K", [(250, 16, 3), (446, 15, 2), (18, 32, 1), (64, 1, 1)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+def test_edge_operator_strips(oracle, n, m, K, prec):
+    """The edge operator in strips of 4 and 8 rows that do not divide the
+    grid (250, 446) and of one row; 7, 15, 16 and 255 columns per tile."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    g = mx.Grid(n, K, kap, FACTORS[:K])
+    x, y = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    ex, ey = mx.Edge(g, m, prec, x), mx.Edge(g, m, prec, y)
+    mx.check(mx.lib().addeval_edge2d_gpu(mx.fz(1.3), mx.fz(0.7), ex.h, ey.h))
+    got = ey.get()
+    for k in range(K):
+        for v in {0, m - 1}:
+            assert rel(got[k, v], oracle.addeval_edge(n, kap, *FACTORS[k], 1.3, 0.7, x[k, v], y[k, v])) < TOL[prec]
