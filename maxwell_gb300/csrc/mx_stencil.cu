@@ -165,11 +165,12 @@ __device__ __forceinline__ cx<R> mx_y(const A& E, R mm, int i, int j) {
 // Measured against a thread per (site, vector), 512^2 cells x 16 vectors:
 // shifted defect, cdd into c64, 8 k-points 1.46 -> 1.03 ms (issue slots 76 %
 // busy; three CTAs per SM, 1.17 ms with two); c64 residual, 32 k-points
-// 1.59 -> 1.46 ms (4.4 TB/s), 64^2 x 12 x 8 k-points 12.6 -> 10.6 us.
+// 1.59 -> 1.50 ms (4.3 TB/s; four CTAs per SM, 1.76 ms with three),
+// 64^2 x 12 x 8 k-points 12.6 -> 11.5 us.
 constexpr int EA_ROWS = 8;
 template <typename R> struct EaShare { static constexpr bool value = sizeof(R) > 4; };
 template <typename SX, typename SY, typename R>
-__global__ void __launch_bounds__(256, 3) k_edge_apply(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap,
+__global__ void __launch_bounds__(256, EaShare<R>::value ? 3 : 4) k_edge_apply(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap,
                                                     Sc axy_s, Sc mm_s, const Sc* __restrict__ mm_kv, Sc cy_s,
                                                     int has_cy, int rj, const SX* __restrict__ x, const SY* yin,
                                                     SY* y) {
