@@ -240,12 +240,11 @@ __global__ void __launch_bounds__(256, EaShare<R>::value ? 3 : 4) k_edge_apply(i
 }
 
 // ------------------------------------------------------------------
-// AFW vertex-patch line Gauss-Seidel.  One thread owns one (k, row, vector)
-// chain and walks its row in the reference's order; rows of one phase touch
-// disjoint unknowns (rows j-1..j+1 read, row j of x and rows j-1, j of y
-// written), so every row of a phase runs concurrently.
-// Local matrix T and its factorisation: see patch_solve in the oracle; the
-// reference's starsolve_common (edge2d.c:2029-2183).
+// AFW vertex-patch line Gauss-Seidel in the reference's order
+// (edge2d.c:2656-3042): rows of one phase touch disjoint unknowns (rows
+// j-1..j+1 of x and j-1, j of y read, row j of x and rows j-1, j of y
+// written), so every row of a phase runs concurrently; along a row the
+// patches follow one another.
 // ------------------------------------------------------------------
 
 // One row of one plane of a (k, vector) edge vector: the row index is
@@ -272,6 +271,15 @@ struct RowIO {
     else if (i >= n) Store<S, R>::st(row + (i - n) * m, conjc(xf) * v);
     else Store<S, R>::st(row + i * m, v);
   }
+};
+// the same for a row and columns inside the unit cell
+template <typename S, typename R>
+struct RowIOI {
+  S* row;
+  int m;
+  __device__ __forceinline__ RowIOI(const RowIO<S, R>& r) : row(r.row), m(r.m) {}
+  __device__ __forceinline__ cx<R> ld(int i) const { return Store<S, R>::ld(row + i * m); }
+  __device__ __forceinline__ void st(int i, cx<R> v) const { Store<S, R>::st(row + i * m, v); }
 };
 template <typename S, typename R>
 __device__ __forceinline__ RowIO<S, R> row_io(S* base, int p, int j, int n, int m, const Seam<R>& seam) {
@@ -446,6 +454,204 @@ __global__ void k_edge_gs_rows(int n, int m, int K, const double* __restrict__ p
       bx1 = bx0; bx0 = nbx; by0 = nby0; by1 = nby1;
       i--;
     }
+  }
+}
+
+// A row's sweep as a linear recurrence.  With the unknowns as they are before
+// a chunk of patches, the correction of patch i alone would be d_i = S_i r_i
+// (S_i the local solve, r_i the four edges' residuals); the patch before it
+// changes three of the values that r_i reads, so
+//   delta_i = d_i + T_i p_{i-1},   p = the previous patch's corrections of
+//                                  the x-edge and the two y-edges they share,
+// with S_i (4 x 4) and T_i (4 x 3) real and made of the four cells' kappa and
+// the scalars alone.  Everything but the recurrence, three FMAs deep per
+// patch, is done by all positions of the chunk at once:
+//   1  every column's weighted curls and x-edge residual (a thread per column
+//      and vector; the column before the chunk as well), and once per segment
+//      of up to 256 columns S_i and T_i (a thread per column), into shared
+//      memory;
+//   2  the patch residuals and d_i = S_i r_i;
+//   3  the recurrence: a lane per (vector, real or imaginary part, unknown),
+//      the three values p from its neighbour lanes;
+//   4  the corrections added to the unknowns in memory.
+// The next chunk starts from the updated unknowns, so nothing is carried
+// over; a chunk holds at most half a row, which keeps the first and the last
+// patch of the row (neighbours across the seam) in different chunks.
+// Without cancellation: S = 1/4 (i0 h0 h0' + i1 h1 h1' + i2 g g' + is8 h3 h3'),
+// h0 = (1,1,1,1), h1 = (1,1,-1,-1), h3 = (1,-1,1,-1), g = (1,-1,-1,1) -
+// l20 h0 - l21 h1, and a cell's weighted curl (of size n^2 x) enters the
+// residuals along a vector e orthogonal to h3: the h3 part, whose factor
+// does not shrink with n, is taken from the residuals without the curls, and
+// S e has none.
+//
+// Bound: FP64 blocks by the FP64 rate (2 FMA per clock and SM, 64 cycles a
+// warp instruction: 141 per patch and vector, against some 260 and five
+// divisions in one thread's chain), small batches by the recurrence.
+// Forward sweeps against a thread per (row, vector) chain: c128, 64^2 one
+// vector 1520 -> 77 us, 128^2 x 16 x 8 k-points 3.54 -> 0.98 ms, 512^2 x 16 x
+// 4 15.1 -> 5.3 ms; float-float 128^2 x 16 x 8 2.12 -> 0.41 ms; c64 64^2 x 12
+// x 8 160 -> 51 us.
+template <typename R> __device__ __forceinline__ R shfl_r(R v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+template <> __device__ __forceinline__ dd shfl_r<dd>(dd v, int src) {
+  return dd_make(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
+}
+
+// the 4 x 4 solve S without its h3 part and the 4 x 3 coupling T of one
+// patch; back: the patch before it in the sweep is the right neighbour
+template <typename R>
+__device__ void afw_patch_matrices(R kLL, R kUL, R kLR, R kUR, R axy, R mm, R s8, R is8, int back, R* S, R* T) {
+  // the factors of afw_factors with three divisions
+  const R one = rc<R>(1.0f), half = rc<R>(0.5f), quarter = rc<R>(0.25f);
+  const R aLL = axy * kLL, aUL = axy * kUL, aLR = axy * kLR, aUR = axy * kUR;
+  const R i0 = one / (aUL + aLR + s8), i1 = one / (aLL + aUR);
+  const R l20 = (aUL - aLR) * i0, l21 = (aLL - aUR) * i1;
+  const R i2 = one / (aLL + aUL + aLR + aUR + s8 - l21 * (aLL - aUR));
+  const R g[4] = {one - l20 - l21, -one - l20 - l21, -one - l20 + l21, one - l20 + l21};
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const R a = ((p < 2) == (q < 2)) ? i0 + i1 : i0 - i1;
+      S[4 * p + q] = quarter * (a + i2 * g[p] * g[q]);
+    }
+  const R s3 = quarter * is8;
+#pragma unroll
+  for (int p = 0; p < 4; p++) {
+    const R h1 = p < 2 ? i1 : -i1;   // i1 h1
+    R lo, up, e1, e2, e3;            // weighted curls' unit responses S e, times kappa
+    if (!back) {
+      lo = aLL * half * (h1 + i2 * (one - l21) * g[p]);
+      up = -(aUL * half * (i0 + i2 * (one - l20) * g[p]));
+      e1 = -lo + up; e2 = -lo; e3 = -up;
+    } else {
+      lo = aLR * half * (i0 - i2 * (one + l20) * g[p]);
+      up = aUR * half * (i2 * (one + l21) * g[p] - h1);
+      e1 = -lo + up; e2 = lo; e3 = up;
+    }
+    const R h3 = (p & 1) ? -s3 : s3;   // the h3 part of S, column 0
+    T[3 * p + 0] = e1 - rc<R>(4.0f) * mm * (back ? S[4 * p + 1] - h3 : S[4 * p] + h3);
+    T[3 * p + 1] = e2 - mm * (S[4 * p + 2] + h3);
+    T[3 * p + 2] = e3 - mm * (S[4 * p + 3] - h3);
+  }
+}
+
+template <typename S, typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_edge_gs_scan(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap,
+                                                      Sc axy_s, Sc mm_s, Sc s8_s, Sc is8_s, int j0, int VB, int P,
+                                                      int SEG, int backward, const S* __restrict__ b, S* x) {
+  // grid (rows of the phase x K, groups of VB vectors); column c = tid / VB
+  // of the chunk, 0 the one before it; P patches per chunk
+  extern __shared__ __align__(16) unsigned char smem_rows[];
+  R* D = reinterpret_cast<R*>(smem_rows);              // [P + 1][VB][2][4] corrections
+  cx<R>* W = reinterpret_cast<cx<R>*>(D + (P + 1) * VB * 8);   // [P + 1][3][VB] curls, x residual
+  R* Sm = reinterpret_cast<R*>(W + (P + 1) * VB * 3);  // [SEG][16]
+  R* Tm = Sm + SEG * 16;                               // [SEG][12]
+  const int tid = threadIdx.x, rows = n / 2, k = blockIdx.x / rows, v0 = blockIdx.y * VB;
+  const int j = j0 + 2 * (int) (blockIdx.x - k * rows);
+  const int c = tid / VB, vv = tid - c * VB, v = v0 + vv < m ? v0 + vv : m - 1;
+  const bool live = v0 + vv < m;
+  Lay L{n, m, K};
+  const Seam<R> seam = seam_load<R>(ph, K, k, n);
+  S* xk = x + L.edge(k, 0, 0, 0, v);
+  S* bk = const_cast<S*>(b) + L.edge(k, 0, 0, 0, v);
+  const RowIO<S, R> X0m = row_io<S, R>(xk, 0, j - 1, n, m, seam), X0c = row_io<S, R>(xk, 0, j, n, m, seam),
+                    X0p = row_io<S, R>(xk, 0, j + 1, n, m, seam), X1m = row_io<S, R>(xk, 1, j - 1, n, m, seam),
+                    X1c = row_io<S, R>(xk, 1, j, n, m, seam), B0c = row_io<S, R>(bk, 0, j, n, m, seam),
+                    B1m = row_io<S, R>(bk, 1, j - 1, n, m, seam), B1c = row_io<S, R>(bk, 1, j, n, m, seam);
+  const R axy = sget<R>(axy_s), mm = sget<R>(mm_s), quarter_is8 = rc<R>(0.25f) * sget<R>(is8_s);
+  const int pq = backward ? 0 : 1;   // the unknown of p that is an x-edge
+  for (int done = 0, seg = 0; done < n;) {
+    // the matrices of the next SEG columns of the sweep, a thread per column
+    if (done == seg) {
+      const int s0 = seg;
+      seg = seg + SEG < n ? seg + SEG : n;
+      for (int q = s0 + tid; q < seg; q += blockDim.x) {
+        const int i = backward ? n - 1 - q : q;
+        afw_patch_matrices<R>(kap(i - 1, j - 1), kap(i - 1, j), kap(i, j - 1), kap(i, j), axy, mm, sget<R>(s8_s),
+                              sget<R>(is8_s), backward, Sm + 16 * (q - s0), Tm + 12 * (q - s0));
+      }
+    }
+    // patches of the chunk at columns i0 .. i0 + np - 1, in memory order;
+    // the matrices of its column c in the segment at at0 + ms c
+    const int np = seg - done < P ? seg - done : P, i0 = backward ? n - done - np : done;
+    const int at0 = (done % SEG) + (backward ? np : -1), ms = backward ? -1 : 1;
+    const int i = i0 + c - 1;
+    const bool col = c <= np, patch = col && c > 0;
+    cx<R> x1, y0, y1, w0, w1, fx, f0, f1;   // f: residuals without the curls
+    // one pass over plain rows where the chunk lies inside the unit cell:
+    // the seam's phase products cost FP64 issue even where no lane needs them
+    const bool inner = j > 0 && j < n - 1 && i0 > 1 && i0 + np < n;
+    auto load = [&](const auto& Xm, const auto& Xc, const auto& Xp, const auto& Ym, const auto& Yc, const auto& Bx,
+                    const auto& Bm, const auto& Bc) {
+      const cx<R> xm = Xm.ld(i), xp = Xp.ld(i), z0 = Ym.ld(i + 1), z1 = Yc.ld(i + 1);
+      x1 = Xc.ld(i);
+      y0 = Ym.ld(i);
+      y1 = Yc.ld(i);
+      w0 = scal(axy * kap(i, j - 1), xm - x1 - y0 + z0);
+      w1 = scal(axy * kap(i, j), x1 - xp - y1 + z1);
+      fx = Bx.ld(i) - scal(mm, times4(x1) + xp + xm);
+      cx<R>* w = W + c * 3 * VB + vv;
+      w[0] = w0; w[VB] = w1; w[2 * VB] = fx;
+      if (patch) {
+        f0 = Bm.ld(i) - scal(mm, times4(y0) + z0 + Ym.ld(i - 1));
+        f1 = Bc.ld(i) - scal(mm, times4(y1) + z1 + Yc.ld(i - 1));
+      }
+    };
+    using RI = RowIOI<S, R>;
+    if (col) {
+      if (inner) load(RI(X0m), RI(X0c), RI(X0p), RI(X1m), RI(X1c), RI(B0c), RI(B1m), RI(B1c));
+      else load(X0m, X0c, X0p, X1m, X1c, B0c, B1m, B1c);
+    }
+    __syncthreads();
+    if (patch) {
+      const cx<R>* w = W + (c - 1) * 3 * VB + vv;
+      const cx<R> fl = w[2 * VB], r0 = fl - (w[VB] - w[0]), r1 = fx - (w1 - w0), r2 = f0 - (w[0] - w0),
+                  r3 = f1 - (w[VB] - w1);
+      const cx<R> h3 = scal(quarter_is8, fl - fx + f0 - f1);
+      const R* Sc = Sm + 16 * (at0 + ms * c);
+      R* d = D + (c * VB + vv) * 8;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        cx<R> t = scal(Sc[4 * q], r0) + scal(Sc[4 * q + 1], r1) + scal(Sc[4 * q + 2], r2) + scal(Sc[4 * q + 3], r3);
+        t = (q & 1) ? t - h3 : t + h3;
+        d[q] = t.re;
+        d[4 + q] = t.im;
+      }
+    }
+    __syncthreads();
+    if (tid < ((8 * VB + 31) & ~31)) {
+      // lane = 8 vector + 4 part + unknown
+      const int q = tid & 3, at = tid < 8 * VB ? tid : 8 * VB - 8 + (tid & 7), quad = (tid & 31) & ~3;
+      const int cc = backward ? np : 1;
+      R cur = D[cc * VB * 8 + at];   // the first patch: delta = d
+      for (int s = 1; s < np; s++) {
+        const int cn = backward ? np - s : 1 + s;
+        const R* t = Tm + 12 * (at0 + ms * cn) + 3 * q;
+        const R dn = D[cn * VB * 8 + at];
+        const R t0 = t[0], t1 = t[1], t2 = t[2];
+        const R p1 = shfl_r(cur, quad + pq), p2 = shfl_r(cur, quad + 2), p3 = shfl_r(cur, quad + 3);
+        cur = dn + t0 * p1 + t1 * p2 + t2 * p3;
+        if (tid < 8 * VB) D[cn * VB * 8 + at] = cur;
+      }
+    }
+    __syncthreads();
+    if (col && live) {
+      const R* d = D + (c * VB + vv) * 8;
+      cx<R> add = czero<R>();
+      if (patch) add = mkc(d[1], d[5]);
+      if (c < np) add += mkc(d[8 * VB], d[8 * VB + 4]);   // the next patch's correction of x(i, j)
+      auto store = [&](const auto& Xc, const auto& Ym, const auto& Yc) {
+        Xc.st(i, x1 + add);
+        if (patch) {
+          Ym.st(i, y0 + mkc(d[2], d[6]));
+          Yc.st(i, y1 + mkc(d[3], d[7]));
+        }
+      };
+      if (inner) store(RI(X0c), RI(X1m), RI(X1c));
+      else store(X0c, X1m, X1c);
+    }
+    __syncthreads();
+    done += np;
   }
 }
 
@@ -1409,17 +1615,43 @@ extern "C" size_t mxk_elem_size(int prec) { return prec == MX_C64 ? 8 : 16; }
    : (prec) == MX_CDD ? F<cdd, dd>(__VA_ARGS__)                        \
    : (int) cudaErrorInvalidValue)
 
+// One phase (the rows j0, j0 + 2, ..) of the row-order smoother.  The
+// recurrence form serves FP64 and float-float blocks of any size; for c64
+// blocks a thread per chain (row, vector, k-point) overtakes it where there
+// are enough chains to hide its latency: forward sweep of 16 vectors, chain
+// against recurrence, 0.55 / 0.40 ms at 32768 chains (128^2, 32 k-points),
+// 2.09 / 1.40 (512^2, 8), 2.18 / 2.02 at 49152 (512^2, 12), 1.15 / 1.37 at
+// 65536 (256^2, 32), 2.30 / 2.63 (512^2, 16).
 template <typename S, typename R>
 static int L_edge_gs_rows(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,
-                          double beta, int j0, int jstep, int nrows, int backward, const void* b,
-                          void* x, cudaStream_t st) {
-  size_t work = (size_t) nrows * m * K;
-  // the tabulated factors serve FP32 sweeps with the scalars they were made for
-  const float4* ftab = (sizeof(R) == 4 && kap.afw && kap.afw_alpha == alpha && kap.afw_beta == beta)
-                           ? (const float4*) kap.afw : nullptr;
-  k_edge_gs_rows<S, R><<<nblocks(work, 64), 64, 0, st>>>(
-      n, m, K, ph, make_kap<R>(kap, n), ftab, make_sc(alpha * (double) n * (double) n), make_sc(beta / 6.0),
-      make_sc(8.0 * beta / 6.0), make_sc(6.0 / (8.0 * beta)), j0, jstep, nrows, backward, (const S*) b, (S*) x);
+                          double beta, int j0, int backward, const void* b, void* x, cudaStream_t st) {
+  const int rows = n / 2;
+  const Sc axy = make_sc(alpha * (double) n * (double) n), mm = make_sc(beta / 6.0), s8 = make_sc(8.0 * beta / 6.0),
+           is8 = make_sc(6.0 / (8.0 * beta));
+  const size_t chains = (size_t) rows * m * K;
+  if constexpr (sizeof(R) == 4) {
+    if (chains >= 57344) {
+      // the tabulated factors serve the scalars they were made for
+      const float4* ftab = (kap.afw && kap.afw_alpha == alpha && kap.afw_beta == beta) ? (const float4*) kap.afw : nullptr;
+      k_edge_gs_rows<S, R><<<nblocks(chains, 64), 64, 0, st>>>(n, m, K, ph, make_kap<R>(kap, n), ftab, axy, mm, s8, is8,
+                                                               j0, 2, rows, backward, (const S*) b, (S*) x);
+      MX_CHECK_LAUNCH();
+      return 0;
+    }
+  }
+  // a CTA takes VB vectors of a row: all of them, or as few as four where
+  // rows x k-points leave SMs without a CTA
+  int VB = m;
+  while (VB > 4 && (size_t) rows * K * ((m + VB - 1) / VB) < 2 * 152) VB = (VB + 1) / 2;
+  int P = 256 / VB - 1;
+  if (P > n / 2) P = n / 2;
+  int threads = ((P + 1) * VB + 31) & ~31;
+  if (threads < ((8 * VB + 31) & ~31)) threads = (8 * VB + 31) & ~31;
+  const int SEG = n < 256 ? n : 256;
+  const size_t smem = sizeof(R) * ((size_t) (P + 1) * VB * 14 + (size_t) SEG * 28);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(k_edge_gs_scan<S, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  k_edge_gs_scan<S, R><<<dim3((unsigned) rows * K, (m + VB - 1) / VB), threads, smem, st>>>(
+      n, m, K, ph, make_kap<R>(kap, n), axy, mm, s8, is8, j0, VB, P, SEG, backward, (const S*) b, (S*) x);
   MX_CHECK_LAUNCH();
   return 0;
 }
@@ -1640,16 +1872,14 @@ extern "C" int mxk_edge_gs_point(int n, int m, int K, const double* ph, mxk_kapp
 extern "C" int mxk_edge_gs(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,
                            double beta, int dir, int prec, const void* b, void* x, mx_stream s) {
   cudaStream_t st = (cudaStream_t) s;
-  int e, half = n / 2;
+  int e;
   if (n & 1) return (int) cudaErrorInvalidValue;
-  if (dir == 0 || dir == 2) {
-    if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, 0, 2, half, 0, b, x, st))) return e;
-    if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, 1, 2, half, 0, b, x, st))) return e;
-  }
-  if (dir == 1 || dir == 2) {
-    if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, 1, 2, half, 1, b, x, st))) return e;
-    if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, 0, 2, half, 1, b, x, st))) return e;
-  }
+  if (dir == 0 || dir == 2)
+    for (int j0 = 0; j0 < 2; j0++)
+      if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, j0, 0, b, x, st))) return e;
+  if (dir == 1 || dir == 2)
+    for (int j0 = 1; j0 >= 0; j0--)
+      if ((e = MX_BY_PREC(prec, L_edge_gs_rows, n, m, K, ph, kap, alpha, beta, j0, 1, b, x, st))) return e;
   return 0;
 }
 

@@ -35,3 +35,24 @@ def test_edge_operator_strips(oracle, n, m, K, prec):
     for k in range(K):
         for v in {0, m - 1}:
             assert rel(got[k, v], oracle.addeval_edge(n, kap, *FACTORS[k], 1.3, 0.7, x[k, v], y[k, v])) < TOL[prec]
+
+
+@pytest.mark.parametrize("n, m, K", [(2, 1, 1), (6, 32, 2), (64, 16, 1), (130, 7, 2), (96, 5, 3)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_row_smoother_chunks(oracle, n, m, K, prec, direction):
+    """The patch smoother in row order: chunks of one patch (n = 2), vectors
+    split over CTAs (one k-point of 16, groups that do not divide 7 or 5),
+    chunks that do not divide the row (130), 32 vectors."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    g = mx.Grid(n, K, kap, FACTORS[:K])
+    b, x = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    eb, ex = mx.Edge(g, m, prec, b), mx.Edge(g, m, prec, x)
+    fn = [mx.lib().gsforward_edge2d_gpu, mx.lib().gsbackward_edge2d_gpu][direction]
+    mx.check(fn(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h))
+    got = ex.get()
+    for k in range(K):
+        for v in {0, m // 2, m - 1}:
+            want = oracle.gs_edge(n, kap, *FACTORS[k], 1.0, 0.8, direction, b[k, v], x[k, v])
+            assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 1e-11)
