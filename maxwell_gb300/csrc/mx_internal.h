@@ -174,6 +174,15 @@ int mxk_rayleigh_ritz(int ns, int m, int K, const double *ga, const double *gm,
                       const int *sel, double drop, double theta_min, double *coef, double *theta,
                       int *info, double *work, mx_stream s);
 
+/* The m lowest eigenpairs above the null space of the coarse pencil (A, M)
+ * for every k (n x n cells, n even, n >= 4, kappa >= 0): the M-normalised
+ * eigenvectors as a block of prec_e (MX_CDD or MX_C128) into E, 1 + lambda
+ * into mu (K*m), info[k] = 0 or -1 where there are fewer than m; work:
+ * mxk_coarse_pairs_work_doubles(n) doubles per k */
+size_t mxk_coarse_pairs_work_doubles(int n);
+int mxk_coarse_pairs(int n, int m, int K, const double *phases, const double *kappa, double *work, int prec_e,
+                     void *E, double *mu, int *info, mx_stream s);
+
 /* Cholesky-QR coefficients: gm (K Hermitian m x m mass Gram matrices) =
  * R^H R, coef = R^{-1} (upper triangular); info[k] = j+1 at a non-positive pivot */
 int mxk_chol_qr_coef(int m, int K, const double *gm, double *coef, int *info, mx_stream s);

@@ -68,7 +68,8 @@ struct mxg_solver {
   int *sel, *info;
   double *cacc;                      /* 4*K*m: plane means of center */
   void *combw;                       /* K*ns*m*16: combine coefficients */
-  double *cA, *cM, *ccoef, *ctheta, *cwork;   /* coarse eigenproblem */
+  int coarse_general;                /* some coarse kappa is negative: solve the pencil of the edge matrices */
+  double *cA, *cM, *ccoef, *ctheta, *cwork;   /* coarse eigenproblem (cA to ctheta: coarse_general only) */
   int *cinfo;
   /* host */
   double *h_ph, *h_stats, *h_mu, *h_res, *h_rq;
@@ -242,6 +243,8 @@ mxg_solver *mxg_solver_new(const mxg_solve_opts *o, const double *kappa_fine)
     }
     free(f); free(p);
   }
+  for(l = 0; l < o->n0 * o->n0; l++)
+    if(!(kk[0][l] >= 0.0)) s->coarse_general = 1;
   for(l = 0; l <= o->L; l++) free(kk[l]);
   for(l = 0; l <= o->L; l++)
     if(dalloc(&s->b[l], elen(s, l) * es_g) || dalloc(&s->x[l], elen(s, l) * es_g) || dalloc(&s->d[l], elen(s, l) * es_g)
@@ -265,11 +268,13 @@ mxg_solver *mxg_solver_new(const mxg_solve_opts *o, const double *kappa_fine)
      || dalloc((void **) &s->rwork, sizeof(double) * mxk_ritz_work_doubles(ns) * K)
      || dalloc((void **) &s->mu, sizeof(double) * m * K) || dalloc((void **) &s->stats, sizeof(double) * NSTAT * m * K)
      || dalloc((void **) &s->sel, sizeof(int) * ns * K) || dalloc((void **) &s->info, sizeof(int) * K)
-     || dalloc((void **) &s->cA, sizeof(double) * 2 * (size_t) N0e * N0e * K)
-     || dalloc((void **) &s->cM, sizeof(double) * 2 * (size_t) N0e * N0e * K)
-     || dalloc((void **) &s->ccoef, sizeof(double) * 2 * (size_t) N0e * N0e * K)
-     || dalloc((void **) &s->ctheta, sizeof(double) * (size_t) N0e * K)
-     || dalloc((void **) &s->cwork, sizeof(double) * mxk_ritz_work_doubles(N0e) * K)
+     || (s->coarse_general
+         && (dalloc((void **) &s->cA, sizeof(double) * 2 * (size_t) N0e * N0e * K)
+             || dalloc((void **) &s->cM, sizeof(double) * 2 * (size_t) N0e * N0e * K)
+             || dalloc((void **) &s->ccoef, sizeof(double) * 2 * (size_t) N0e * N0e * K)
+             || dalloc((void **) &s->ctheta, sizeof(double) * (size_t) N0e * K)))
+     || dalloc((void **) &s->cwork, sizeof(double) * K
+               * (s->coarse_general ? mxk_ritz_work_doubles(N0e) : mxk_coarse_pairs_work_doubles(o->n0)))
      || dalloc((void **) &s->cinfo, sizeof(int) * K)
      || dalloc((void **) &s->cacc, sizeof(double) * 4 * K * m)
      || dalloc(&s->combw, (size_t) 16 * ns * m * K))
@@ -832,15 +837,15 @@ static int iterate(mxg_solver *s, int l, int maxsteps, int K_active)
   return 0;
 }
 
-/* coarse generalized eigenproblem (exp_bloch2d.c:530-554) and the nested
- * iteration (exp_bloch2d.c:562-732) for every k of the wave */
-static int cold_start(mxg_solver *s, int K_active)
+/* The coarse eigenproblem (exp_bloch2d.c:530-554) as the pencil of the edge
+ * matrices: only where a coarse kappa is negative and the cell form
+ * (mxk_coarse_pairs) does not exist */
+static int coarse_pencil(mxg_solver *s)
 {
-  int N = 2 * s->n0 * s->n0, m = s->m, K = s->K, k, i, v, l;
+  int N = 2 * s->n0 * s->n0, m = s->m, K = s->K, k, i, v;
   double *th = malloc(sizeof(double) * N * K), *cf = malloc(sizeof(double) * 2 * (size_t) N * N * K);
   double *e0 = malloc(sizeof(double) * 2 * (size_t) K * N * m);
   int e = 0;
-  double t0 = now_s();
   L_(mxk_dense_edge(s->n0, K, s->ph, kap(s, 0), 1.0, 0.0, s->cA, s->st));
   L_(mxk_dense_edge(s->n0, K, s->ph, kap(s, 0), 0.0, 1.0, s->cM, s->st));
   L_(mxk_rayleigh_ritz(N, N, K, s->cA, s->cM, 0, 1e-14, -1e300, s->ccoef, s->ctheta, s->cinfo, s->cwork, s->st));
@@ -848,7 +853,6 @@ static int cold_start(mxg_solver *s, int K_active)
   if(!e) e = (int) cudaMemcpyAsync(cf, s->ccoef, sizeof(double) * 2 * (size_t) N * N * K, cudaMemcpyDeviceToHost, s->st);
   if(!e) e = (int) cudaStreamSynchronize(s->st);
   if(e) { free(th); free(cf); free(e0); return e; }
-  if(s->timing) fprintf(stderr, "  coarse eigenproblem %.3f s\n", now_s() - t0);
   /* skip |lambda| < 1e-8 (exp_bloch2d.c:546-551); level-0 block layout of
    * one k is row-major N x m */
   for(k = 0; k < K; k++) {
@@ -883,7 +887,26 @@ static int cold_start(mxg_solver *s, int K_active)
   }
   free(th); free(cf); free(e0);
   if(e) return e;
-  TRY(upload_mu(s));
+  return upload_mu(s);
+}
+
+/* coarse eigenproblem (exp_bloch2d.c:530-554) and the nested iteration
+ * (exp_bloch2d.c:562-732) for every k of the wave */
+static int cold_start(mxg_solver *s, int K_active)
+{
+  int m = s->m, K = s->K, k, l;
+  double t0 = now_s();
+  if(s->coarse_general)
+    TRY(coarse_pencil(s));
+  else {
+    L_(mxk_coarse_pairs(s->n0, m, K, s->ph, s->kd[0], s->cwork, s->pe, s->E, s->mu, s->cinfo, s->st));
+    TRY((int) cudaMemcpyAsync(s->h_info, s->cinfo, sizeof(int) * K, cudaMemcpyDeviceToHost, s->st));
+    TRY((int) cudaMemcpyAsync(s->h_mu, s->mu, sizeof(double) * m * K, cudaMemcpyDeviceToHost, s->st));
+    TRY((int) cudaStreamSynchronize(s->st));
+    for(k = 0; k < K; k++)
+      if(s->h_info[k]) return MXG_ECONV;
+  }
+  if(s->timing) fprintf(stderr, "  coarse eigenproblem %.3f s\n", now_s() - t0);
   for(l = 1; l <= s->L; l++) {
     L_(mxk_zero(s->pe, s->En, elen(s, l), s->st));
     L_(mxk_edge_prolong(s->n[l - 1], m, K, s->ph, 1.0, s->pe, s->E, s->En, s->st));

@@ -56,3 +56,21 @@ def test_row_smoother_chunks(oracle, n, m, K, prec, direction):
         for v in {0, m // 2, m - 1}:
             want = oracle.gs_edge(n, kap, *FACTORS[k], 1.0, 0.8, direction, b[k, v], x[k, v])
             assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 1e-11)
+
+
+@pytest.mark.parametrize("n0, L, m", [(4, 2, 6), (6, 2, 9), (10, 1, 12), (12, 1, 8)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_coarse_grid_sizes(oracle, n0, L, m, precision):
+    """Solves that start from coarse grids of 16, 36 (matrices in shared
+    memory), 100 and 144 cells (in global memory), Gamma among the k-points."""
+    rng = np.random.default_rng(n0)
+    n = n0 << L
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac, ie = FACTORS, (2 * m) // 3
+    s = mx.Solver(kap, n0=n0, L=L, ieigs=ie, m=m, method=1, precision=precision, max_nested=40, max_steps=60,
+                  wave=len(fac), relative=0, tol=1e-8)
+    lam, _, res = s.solve(fac)
+    st, lam_o, _, _, _ = oracle.bloch_solve(kap, fac, n0=n0, L=L, ieigs=ie, m=m, method=1, max_nested=40,
+                                            max_steps=60, tol=1e-8, relative=0, extrapolation="n", wave=len(fac))
+    assert st == 0 and res[:, :ie].max() <= 1e-8
+    assert np.abs(lam[:, :ie] - lam_o[:, :ie]).max() / lam_o[:, :ie].max() < 1e-8
