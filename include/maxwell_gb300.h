@@ -215,6 +215,8 @@ int restriction_node2d_gpu(mxg_field alpha, const node2d_gpu *f, node2d_gpu *c);
 int residual_restriction_node2d_gpu(mxg_field alpha, const node2d_gpu *b, const node2d_gpu *x, node2d_gpu *c);
 int gradient_node2d_gpu(mxg_field alpha, const node2d_gpu *x, edge2d_gpu *y);
 int adjgradient_node2d_gpu(mxg_field alpha, const edge2d_gpu *x, node2d_gpu *y);
+/* vcycle_node2d (node2d.c:1352-1389); b[l], x[l], d[l] below level L and
+ * d[L] are work space (their contents after the call are not defined) */
 int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x,
                       node2d_gpu **d);
 int densematrix_node2d_gpu(int fixnull, const grid2d_gpu *gr, matrix_gpu *a);

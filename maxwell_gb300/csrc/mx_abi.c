@@ -641,20 +641,54 @@ int adjgradient_node2d_gpu(mxg_field alpha, const edge2d_gpu *x, node2d_gpu *y)
   return mxk_adjgradient(g->n, x->m, g->K, g->ph, creal_(alpha), 0, 1.0, x->prec, x->d, y->prec, y->d, g->st);
 }
 
+/* The level from which vcycle_node2d_gpu runs in one launch (0: none): a
+ * coarse inverse, grids that halve from level to level with the same Bloch
+ * factors, vectors of one shape and precision. */
+static int fused_level_n(int L, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x)
+{
+  const grid2d_gpu *g0 = x[0]->gr;
+  int c, l;
+  if(!Ac || !Ac->factored || Ac->rows != g0->n * g0->n || Ac->K != g0->K) return 0;
+  c = mxk_node_vcycle_top(g0->n, L, x[0]->prec);
+  for(l = 0; l <= c; l++) {
+    const grid2d_gpu *g = x[l]->gr;
+    if(g->n != g0->n << l || g->K != g0->K || memcmp(g->h_ph, g0->h_ph, sizeof(double) * 4 * g0->K)
+       || x[l]->m != x[0]->m || x[l]->prec != x[0]->prec || b[l]->m != x[0]->m || b[l]->prec != x[0]->prec
+       || b[l]->gr->n != g->n || b[l]->gr->K != g->K)
+      return 0;
+  }
+  return c;
+}
+
+/* one sweep of a V-cycle: gs_n without its synchronisation where the sweep
+ * needs no scratch vector */
+static int gs_cycle(const node2d_gpu *b, node2d_gpu *x, int dir)
+{
+  const grid2d_gpu *g = x->gr;
+  if(b->prec != x->prec || b->m != x->m) return MXG_EINVAL;
+  if(mxk_node_gs_oop_ok(g->n, x->m, x->prec)) return gs_n(1.0, b, x, dir);
+  return mxk_node_gs(g->n, x->m, g->K, g->ph, 1.0, dir, x->prec, b->d, x->d, g->st);
+}
+
 int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
 {
-  int l, i;
-  for(l = L; l > 0; l--) {
+  int l, i, lc = fused_level_n(L, Ac, b, x);
+  for(l = L; l > lc; l--) {
     const grid2d_gpu *g = x[l]->gr;
     for(i = 0; i < nu; i++)
-      TRY(gs_n(1.0, b[l], x[l], 0));
+      TRY(gs_cycle(b[l], x[l], 0));
     if(b[l]->prec != d[l]->prec) return MXG_EINVAL;
     TRY(mxk_node_apply(g->n, x[l]->m, g->K, g->ph, -1.0, 1.0, x[l]->prec, x[l]->d, b[l]->d, d[l]->d, g->st));
     TRY(zero_node2d_gpu(b[l - 1]));
     TRY(mxk_node_restrict(g->n / 2, x[l]->m, g->K, g->ph, 1.0, d[l]->prec, d[l]->d, b[l - 1]->d, g->st));
-    TRY(zero_node2d_gpu(x[l - 1]));
+    if(l - 1 > lc || lc == 0) TRY(zero_node2d_gpu(x[l - 1]));
   }
-  if(Ac) {
+  if(lc > 0) {
+    const grid2d_gpu *g = x[lc]->gr;
+    TRY(mxk_node_vcycle(x[0]->gr->n, lc, x[lc]->m, g->K, nu, 1, lc < L, g->ph, Ac->d, 0, x[lc]->prec, b[lc]->d,
+                        x[lc]->d, g->st));
+  }
+  else if(Ac) {
     const grid2d_gpu *g = x[0]->gr;
     if(!Ac->factored || Ac->rows != g->n * g->n || Ac->K != g->K) return MXG_EINVAL;
     TRY(mxk_coarse_apply(Ac->rows, x[0]->m, g->K, Ac->d, 0, x[0]->prec, b[0]->d, x[0]->d, g->st));
@@ -662,11 +696,11 @@ int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2
   else
     for(i = 0; i < nu; i++)
       TRY(gs_n(1.0, b[0], x[0], 2));
-  for(l = 1; l <= L; l++) {
+  for(l = lc + 1; l <= L; l++) {
     const grid2d_gpu *g = x[l]->gr;
     TRY(mxk_node_prolong(g->n / 2, x[l]->m, g->K, g->ph, 1.0, x[l]->prec, x[l - 1]->d, x[l]->d, g->st));
     for(i = 0; i < nu; i++)
-      TRY(gs_n(1.0, b[l], x[l], 1));
+      TRY(gs_cycle(b[l], x[l], 1));
   }
   return (int) cudaStreamSynchronize(x[L]->gr->st);
 }

@@ -103,6 +103,13 @@ void mxk_node_gs_oop_get_shape(int *strip, int *band);
  * 2^log2 (coarse node, vector, k-point) triples on (0 .. 62) */
 int mxk_node_rr_set_strips(int log2);
 int mxk_node_rr_get_strips(void);
+/* whole V-cycles of the levels n0 .. n0 << top (nu sweeps each way, the
+ * coarse inverse ainv) in one launch: `cycles` of them on b, x of the top
+ * level, x starting from zero where zero is set.  mxk_node_vcycle_top: the
+ * highest level up to `top` that this form takes (0: none) */
+int mxk_node_vcycle_top(int n0, int top, int prec);
+int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, const double *phases,
+                    const double *ainv, const void *ainv_c64, int prec, const void *b, void *x, mx_stream s);
 int mxk_node_prolong(int nc, int m, int K, const double *phases, double alpha,
                      int prec, const void *c, void *f, mx_stream s);
 int mxk_node_restrict(int nc, int m, int K, const double *phases, double alpha,

@@ -460,19 +460,37 @@ static int vcycle_e(mxg_solver *s, int top)
   return 0;
 }
 
+/* The level from which the node V-cycle runs in one launch (0: none; with
+ * profiling on, the finest level keeps its launches, which carry the events). */
+static int fused_node_level(const mxg_solver *s, int top)
+{
+  int c = mxk_node_vcycle_top(s->n0, top, s->pg);
+  return s->prof && c == s->L ? 0 : c;
+}
+
+static int fused_node_cycles(mxg_solver *s, int l, int cycles, int zero)
+{
+  L_(mxk_node_vcycle(s->n0, l, s->m, s->K, s->o.smoother_steps, cycles, zero, s->ph, s->an_inv, s->an_inv_f, s->pg,
+                     s->bg[l], s->xg[l], s->st));
+  return 0;
+}
+
 /* vcycle_node2d (node2d.c:1352-1389) on bg[top], xg[top] */
 static int vcycle_n(mxg_solver *s, int top)
 {
-  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg;
-  for(l = top; l > 0; l--) {
+  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg, lc = fused_node_level(s, top);
+  for(l = top; l > lc; l--) {
     int n = s->n[l];
     TRY(node_smooth(s, l, 0, nu));
     /* the residual and its restriction in one kernel (written, not added) */
     L_(mxk_node_residual_restrict(n / 2, m, K, s->ph, 1.0, pg, s->xg[l], s->bg[l], s->bg[l - 1], s->st));
-    L_(mxk_zero(pg, s->xg[l - 1], nlen(s, l - 1), s->st));
+    if(l - 1 > lc || lc == 0) L_(mxk_zero(pg, s->xg[l - 1], nlen(s, l - 1), s->st));
   }
-  L_(mxk_coarse_apply(s->n0 * s->n0, m, K, s->an_inv, s->an_inv_f, pg, s->bg[0], s->xg[0], s->st));
-  for(l = 1; l <= top; l++) {
+  if(lc > 0)
+    TRY(fused_node_cycles(s, lc, 1, lc < top));
+  else
+    L_(mxk_coarse_apply(s->n0 * s->n0, m, K, s->an_inv, s->an_inv_f, pg, s->bg[0], s->xg[0], s->st));
+  for(l = lc + 1; l <= top; l++) {
     int n = s->n[l];
     L_(mxk_node_prolong(n / 2, m, K, s->ph, 1.0, pg, s->xg[l - 1], s->xg[l], s->st));
     TRY(node_smooth(s, l, 1, nu));
@@ -520,6 +538,7 @@ static int run_graphed(mxg_solver *s, int l, cudaGraphExec_t *exec, long *nlaunc
 static int lift_body(mxg_solver *s, int l)
 {
   int i;
+  if(l > 0 && fused_node_level(s, l) == l) return fused_node_cycles(s, l, s->o.gradient_steps, 1);
   L_(mxk_zero(s->pg, s->xg[l], nlen(s, l), s->st));
   for(i = 0; i < s->o.gradient_steps; i++)
     TRY(vcycle_n(s, l));

@@ -74,3 +74,50 @@ def test_coarse_grid_sizes(oracle, n0, L, m, precision):
                                             max_steps=60, tol=1e-8, relative=0, extrapolation="n", wave=len(fac))
     assert st == 0 and res[:, :ie].max() <= 1e-8
     assert np.abs(lam[:, :ie] - lam_o[:, :ie]).max() / lam_o[:, :ie].max() < 1e-8
+
+
+@pytest.mark.parametrize("n0, L, m, K", [(4, 1, 1, 1), (8, 3, 3, 2), (10, 2, 2, 1), (6, 4, 1, 2), (8, 4, 2, 1)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+def test_node_vcycle_levels(oracle, n0, L, m, K, prec):
+    """Node V-cycles from a given start on grids that run in one launch down
+    to the coarse solve (8, 64, 40 and 96 nodes a side: one, two and three
+    positions per lane, rows shorter than the warp; in FP64 96 and 128 keep
+    upper levels of their own) against the cycle put together from the
+    oracle's sweeps, residual and transfers."""
+    rng = np.random.default_rng(n0 + L)
+    n = n0 << L
+    fac = FACTORS[[0, 2]][:K]
+    grids = [mx.Grid(n, K, None, fac)]
+    for _ in range(L):
+        grids.append(grids[-1].coarsen())
+    grids = grids[::-1]
+    import ctypes as C
+    b, x, d = ([mx.Node(g, m, prec) for g in grids] for _ in range(3))
+    rhs, start = cv(rng, K, m, n * n), cv(rng, K, m, n * n)
+    b[L].put(rhs)
+    x[L].put(start)
+    rhs, start = b[L].get(), x[L].get()   # as stored
+    A, info = mx.Matrix(n0 * n0, K), np.zeros(K, np.int32)
+    mx.check(mx.lib().densematrix_node2d_gpu(1, grids[0].h, A.h))
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    arr = [(C.c_void_p * (L + 1))(*[o.h for o in objs]) for objs in (b, x, d)]
+    mx.check(mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr))
+    got = x[L].get()
+
+    def cycle(l, f, bl, xl):
+        nl = n0 << l
+        if l == 0:
+            return np.linalg.solve(oracle.dense_node(n0, *f, 1), bl)
+        for _ in range(2):
+            xl = oracle.gs_node(nl, *f, 1.0, 0, bl, xl)
+        r = oracle.addeval_node(nl, *f, -1.0, xl, bl)
+        c = oracle.restrict_node(nl // 2, *f, 1.0, r, np.zeros(nl * nl // 4, complex))
+        xl = oracle.prolong_node(nl // 2, *f, 1.0, cycle(l - 1, f, c, np.zeros_like(c)), xl)
+        for _ in range(2):
+            xl = oracle.gs_node(nl, *f, 1.0, 1, bl, xl)
+        return xl
+
+    # the sweeps' tolerances (2e-5 and 1e-11) over the cycle's coarse solve
+    for k in range(K):
+        for v in range(m):
+            assert rel(got[k, v], cycle(L, fac[k], rhs[k, v], start[k, v])) < (1e-4 if prec == mx.C64 else 1e-10)
