@@ -817,8 +817,7 @@ int mxg_device_ok(void)
   return n > 0;
 }
 
-/* accessors for the solver translation unit */
-const double *mxg__grid_phases(const grid2d_gpu *g) { return g->ph; }
+/* the device storage of an edge batch */
 void *mxg__edge_data(const edge2d_gpu *e) { return e->d; }
 
 /* ------------------------------------------------------------------ */

@@ -680,29 +680,47 @@ static size_t combine_tiled_smem() {
 }
 
 // ------------------------------------------------------------------
-// sensitivity: grad[c] = -n^2 kappa_c^2 sum_{k,v} w_kv |curl_c e_kv|^2
+// sensitivity: grad[c] = -n^2 kappa_c^2 sum_{k,v} w_kv |curl_c e_kv|^2, the
+// eigenvectors in the dense order [k][v][plane][j][i] in which callers hold
+// them.  A thread takes a cell and a share of the k-points; the shares' sums
+// are added in a fixed order.  Bound by the transfer of the eigenvectors from
+// the host; the kernel by FP64 issue (128^2 cells, 24 k-points x 9 vectors:
+// 0.144 ms, 0.46 ms with one thread per cell).
 // ------------------------------------------------------------------
-template <typename S, typename R>
-__global__ void k_eps_sensitivity(int n, int m, int K, const double* __restrict__ ph,
-                                  const double* __restrict__ kappa, const double* __restrict__ w,
-                                  const S* __restrict__ e, double* __restrict__ grad) {
-  size_t c = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= (size_t) n * n) return;
-  int i = (int) (c % n), j = (int) (c / n);
-  Lay L{n, m, K};
+__global__ void k_eps_curls(int n, int m, int K, int per, const double* __restrict__ ph,
+                            const double* __restrict__ w, const double2* __restrict__ e, double* __restrict__ part) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, nn = n * n;
+  if (c >= nn) return;
+  const int i = c % n, j = c / n, k0 = blockIdx.y * per, k1 = k0 + per < K ? k0 + per : K;
+  const bool si = i == n - 1, sj = j == n - 1;
+  const int right = si ? c - i : c + 1, up = sj ? i : c + n;
   double s = 0.0;
-  for (int k = 0; k < K; k++) {
-    Seam<R> sm = seam_load<R>(ph, K, k, n);
+  for (int k = k0; k < k1; k++) {
+    const Seam<double> sm = seam_load<double>(ph, K, k, n);
+#pragma unroll 4
     for (int v = 0; v < m; v++) {
-      double wv = w[(size_t) k * m + v];
+      const double wv = w[(size_t) k * m + v];
+      const double2* ex = e + ((size_t) k * m + v) * 2 * nn;
+      const double2* ey = ex + nn;
       if (wv == 0.0) continue;
-      EA<S, R> E{e + L.edge(k, 0, 0, 0, v), n, m, sm};
-      cx<R> cu = curlc<R>(E, i, j);
-      double re = Real<R>::to_double(cu.re), im = Real<R>::to_double(cu.im);
+      const double2 x0 = ex[c], y0 = ey[c];
+      double2 x1 = ex[up], y1 = ey[right];
+      if (sj) x1 = make_double2(sm.yf.re * x1.x - sm.yf.im * x1.y, sm.yf.re * x1.y + sm.yf.im * x1.x);
+      if (si) y1 = make_double2(sm.xf.re * y1.x - sm.xf.im * y1.y, sm.xf.re * y1.y + sm.xf.im * y1.x);
+      const double re = x0.x - x1.x - y0.x + y1.x, im = x0.y - x1.y - y0.y + y1.y;
       s += wv * (re * re + im * im);
     }
   }
-  double kc = kappa[c];
+  part[(size_t) blockIdx.y * nn + c] = s;
+}
+
+__global__ void k_eps_gradient(int n, int parts, const double* __restrict__ kappa, const double* __restrict__ part,
+                               double* __restrict__ grad) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, nn = n * n;
+  if (c >= nn) return;
+  double s = 0.0;
+  for (int q = 0; q < parts; q++) s += part[(size_t) q * nn + c];
+  const double kc = kappa[c];
   grad[c] = -(double) n * n * kc * kc * s;
 }
 
@@ -1195,14 +1213,22 @@ extern "C" int mxk_select_columns(int ns, int m, int K, const double* stats, con
   return 0;
 }
 
+// shares of the k-points: enough for about four CTAs per SM
+extern "C" int mxk_eps_sensitivity_parts(int n, int K) {
+  const int blocks = (n * n + 255) / 256;
+  const int want = (4 * sm_count() + blocks - 1) / blocks;
+  const int per = (K + want - 1) / want > 1 ? (K + want - 1) / want : 1;
+  return (K + per - 1) / per;
+}
+
 extern "C" int mxk_eps_sensitivity(int n, int m, int K, const double* ph, const double* kappa, const double* w,
-                                   int pe, const void* e, double* grad, mx_stream s) {
-  size_t nc = (size_t) n * n;
-  dim3 g((unsigned) ((nc + 255) / 256)), b(256);
+                                   const void* e, double* part, double* grad, mx_stream s) {
+  const int parts = mxk_eps_sensitivity_parts(n, K), per = (K + parts - 1) / parts;
+  const unsigned blocks = (unsigned) (((size_t) n * n + 255) / 256);
   cudaStream_t st = (cudaStream_t) s;
-  if (pe == MX_CDD) k_eps_sensitivity<cdd, dd><<<g, b, 0, st>>>(n, m, K, ph, kappa, w, (const cdd*) e, grad);
-  else if (pe == MX_C128) k_eps_sensitivity<double2, double><<<g, b, 0, st>>>(n, m, K, ph, kappa, w, (const double2*) e, grad);
-  else k_eps_sensitivity<float2, float><<<g, b, 0, st>>>(n, m, K, ph, kappa, w, (const float2*) e, grad);
+  k_eps_curls<<<dim3(blocks, parts), 256, 0, st>>>(n, m, K, per, ph, w, (const double2*) e, part);
+  MX_CHECK_LAUNCH();
+  k_eps_gradient<<<blocks, 256, 0, st>>>(n, parts, kappa, part, grad);
   MX_CHECK_LAUNCH();
   return 0;
 }

@@ -223,15 +223,16 @@ int mxk_block_combine(int n, int m, int K, int nb, const int *precs, const void 
  * above tol: the columns of the Ritz basis under soft locking */
 int mxk_select_columns(int ns, int m, int K, const double *stats, const double *mu, double tol,
                        int relative, int all, int *sel, mx_stream s);
-/* per-cell eigenvalue sensitivity: grad[c] = -n^2 kappa_c^2 sum_{k,v} w[k*m+v] |curl_c e|^2 */
+/* per-cell eigenvalue sensitivity: grad[c] = -n^2 kappa_c^2 sum_{k,v} w[k*m+v] |curl_c e|^2;
+ * e in the dense order [k][v][2n^2] (complex double), part:
+ * mxk_eps_sensitivity_parts(n, K) * n^2 doubles of scratch */
+int mxk_eps_sensitivity_parts(int n, int K);
 int mxk_eps_sensitivity(int n, int m, int K, const double *phases, const double *kappa,
-                        const double *weights, int prec_e, const void *e, double *grad,
+                        const double *weights, const void *e, double *part, double *grad,
                         mx_stream s);
 
-/* accessors of the public handles (mx_abi.c) */
-struct grid2d_gpu;
+/* the device storage of a public handle (mx_abi.c) */
 struct edge2d_gpu;
-const double *mxg__grid_phases(const struct grid2d_gpu *g);
 void *mxg__edge_data(const struct edge2d_gpu *e);
 
 #ifdef __cplusplus

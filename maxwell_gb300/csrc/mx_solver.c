@@ -1373,27 +1373,36 @@ int mxg_solver_kernel_time(mxg_solver *s, int which, double *ms, long *count, do
 int mxg_eps_sensitivity(int n, const double *kappa, int nk, const mxg_field *xf, const mxg_field *yf, int m,
                         const mxg_field *evec, const double *weights, double *grad)
 {
-  grid2d_gpu *g;
-  edge2d_gpu *e;
-  double *dk, *dw, *dg;
-  int err;
+  /* one device buffer: eigenvectors in the caller's order, kappa, weights,
+   * phase table, partial sums, gradient */
+  size_t nn, ne, off[6], bytes;
+  double *d, *tab;
+  int err, k;
   if(m < 1 || m > 32) return MXG_EINVAL;
-  g = new_grid2d_gpu(n, n, 1.0 / n, 1.0 / n, nk);
-  if(!g) return MXG_ENOMEM;
-  err = setkappa_grid2d_gpu(g, kappa);
-  if(!err) err = setbloch_grid2d_gpu(g, xf, yf);
-  e = err ? 0 : new_edge2d_gpu(g, m, MXG_C128);
-  if(!e) { del_grid2d_gpu(g); return err ? err : MXG_ENOMEM; }
-  err = denseto_edge2d_gpu(evec, e);
-  if(cudaMalloc((void **) &dk, sizeof(double) * n * n)) { del_edge2d_gpu(e); del_grid2d_gpu(g); return MXG_ENOMEM; }
-  if(cudaMalloc((void **) &dw, sizeof(double) * nk * m)) { cudaFree(dk); del_edge2d_gpu(e); del_grid2d_gpu(g); return MXG_ENOMEM; }
-  if(cudaMalloc((void **) &dg, sizeof(double) * n * n)) { cudaFree(dk); cudaFree(dw); del_edge2d_gpu(e); del_grid2d_gpu(g); return MXG_ENOMEM; }
-  if(!err) err = (int) cudaMemcpy(dk, kappa, sizeof(double) * n * n, cudaMemcpyHostToDevice);
-  if(!err) err = (int) cudaMemcpy(dw, weights, sizeof(double) * nk * m, cudaMemcpyHostToDevice);
-  if(!err) err = mxk_eps_sensitivity(n, m, nk, mxg__grid_phases(g), dk, dw, MX_C128, mxg__edge_data(e), dg, 0);
-  if(!err) err = (int) cudaMemcpy(grad, dg, sizeof(double) * n * n, cudaMemcpyDeviceToHost);
-  cudaFree(dk); cudaFree(dw); cudaFree(dg);
-  del_edge2d_gpu(e);
-  del_grid2d_gpu(g);
+  if(n < 2 || (n & 1) || nk < 1) return MXG_ENOMEM;   /* (no grid of that shape) */
+  nn = (size_t) n * n;
+  ne = (size_t) nk * m * 2 * nn;
+  off[0] = 2 * ne;
+  off[1] = off[0] + nn;
+  off[2] = off[1] + (((size_t) nk * m + 1) & ~(size_t) 1);
+  off[3] = off[2] + mxk_phase_bytes(nk) / sizeof(double);
+  off[4] = off[3] + mxk_eps_sensitivity_parts(n, nk) * nn;
+  bytes = sizeof(double) * (off[4] + nn);
+  tab = malloc(mxk_phase_bytes(nk));
+  if(!tab) return MXG_ENOMEM;
+  if(cudaMalloc((void **) &d, bytes)) { cudaGetLastError(); free(tab); return MXG_ENOMEM; }
+  for(k = 0; k < nk; k++) {
+    tab[4 * k] = creal(xf[k]); tab[4 * k + 1] = cimag(xf[k]);
+    tab[4 * k + 2] = creal(yf[k]); tab[4 * k + 3] = cimag(yf[k]);
+  }
+  mxk_phase_fill(nk, tab);
+  err = (int) cudaMemcpy(d, evec, sizeof(double) * 2 * ne, cudaMemcpyHostToDevice);
+  if(!err) err = (int) cudaMemcpy(d + off[0], kappa, sizeof(double) * nn, cudaMemcpyHostToDevice);
+  if(!err) err = (int) cudaMemcpy(d + off[1], weights, sizeof(double) * nk * m, cudaMemcpyHostToDevice);
+  if(!err) err = (int) cudaMemcpy(d + off[2], tab, mxk_phase_bytes(nk), cudaMemcpyHostToDevice);
+  if(!err) err = mxk_eps_sensitivity(n, m, nk, d + off[2], d + off[0], d + off[1], d, d + off[3], d + off[4], 0);
+  if(!err) err = (int) cudaMemcpy(grad, d + off[4], sizeof(double) * nn, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  free(tab);
   return err;
 }

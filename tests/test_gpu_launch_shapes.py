@@ -121,3 +121,17 @@ def test_node_vcycle_levels(oracle, n0, L, m, K, prec):
     for k in range(K):
         for v in range(m):
             assert rel(got[k, v], cycle(L, fac[k], rhs[k, v], start[k, v])) < (1e-4 if prec == mx.C64 else 1e-10)
+
+
+@pytest.mark.parametrize("n, K, m", [(2, 1, 1), (30, 40, 3), (126, 5, 32)])
+def test_sensitivity_shares(oracle, n, K, m):
+    """The permittivity gradient with one, several and all k-points per
+    share of the reduction, zero weights among them."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(-3, 3, (K, 2)))
+    vec, w = cv(rng, K, m, 2 * n * n), rng.standard_normal((K, m))
+    w[0, 0] = 0.0
+    got = mx.eps_sensitivity(n, kap, fac, vec, w)
+    want = sum(oracle.eps_sensitivity(n, kap, *fac[k], vec[k], w[k]) for k in range(K))
+    assert rel(got, want) < 1e-12
