@@ -248,36 +248,74 @@ __device__ __forceinline__ cx<float> ld_any_f(int prec, const void* base, size_t
   return Store<double2, float>::ld((const double2*) base + off);
 }
 
+// an entry (i, j) of the partial sums from its accumulated parts q: A + M =
+// axy * (sum over cells of kappa conj(curl_i) curl_j) + M, or for the residual
+// form of the cross entries theta_j * M + s_i^H r_j
+__device__ __forceinline__ void gram_entry(const GramArgs& a, int k, int e, int i, int j, int mh, bool use_r, double axy,
+                                           const double* q, double* out) {
+  double* o = out + (size_t) e * 4;
+  if (use_r && i >= mh && j < mh) {
+    const double th = a.theta[(size_t) k * a.m + j];
+    o[0] = th * q[2] + q[0];
+    o[1] = th * q[3] + q[1];
+  } else {
+    o[0] = axy * q[0] + q[2];
+    o[1] = axy * q[1] + q[3];
+  }
+  o[2] = q[2];
+  o[3] = q[3];
+}
+
+// (re, im) += conj(a) b
+template <typename R> __device__ __forceinline__ void gram_mac(cx<R>& s, cx<R> a, cx<R> b) { s += conjc(a) * b; }
+template <> __device__ __forceinline__ void gram_mac<double>(cx<double>& s, cx<double> a, cx<double> b) {
+  s.re = fma(a.re, b.re, fma(a.im, b.im, s.re));
+  s.im = fma(a.re, b.im, fma(-a.im, b.re, s.im));
+}
+
+template <typename HI> struct HiStore;
+template <> struct HiStore<dd> { using T = cdd; };
+template <> struct HiStore<double> { using T = double2; };
+
 // HI = dd for the mixed solver (column block 0 is cdd, the other blocks c64),
-// double for the plain solver (every block c128, every column high).
-template <typename HI>
-__global__ void k_block_gram(GramArgs a, int mh, int ebase) {
+// double for the plain solver.  ALLHI: every column is high (c128 blocks);
+// the FP32 accumulators and staging do not exist then.  FP64 blocks are bound
+// by the FP64 rate: the site's kappa goes into the staged curl of column j
+// (component 5), entries are pure multiply-adds, and the threads without an
+// entry of their own share the sites.  11 c128 vectors, 120^2, 5 k-points:
+// 0.51 -> 0.26 ms.
+template <typename HI, bool ALLHI>
+__global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int ebase) {
   int k = blockIdx.y, chunk = blockIdx.x;
   int n = a.n, m = a.m, ns = a.ns;
   int nent = ns * (ns + 1) / 2;
   Lay L{n, m, a.K};
   extern __shared__ double smd[];
   // staging per site and column: curl, x, y, (Mx), (My)
-  cx<HI>* hi = reinterpret_cast<cx<HI>*>(smd);                        // TS*mh*5
-  cx<float>* lo = reinterpret_cast<cx<float>*>(hi + TS * mh * 5);      // TS*ns*5
-  HI* kap_h = reinterpret_cast<HI*>(lo + TS * ns * 5);                // TS
-  float* kap_t = reinterpret_cast<float*>(kap_h + TS);                // TS
+  cx<HI>* hi = reinterpret_cast<cx<HI>*>(smd);                        // TS*mh*6
+  cx<float>* lo = reinterpret_cast<cx<float>*>(hi + TS * mh * 6);      // TS*ns*5 (not ALLHI)
+  float* kap_t = reinterpret_cast<float*>(lo + (ALLHI ? 0 : TS * ns * 5));   // TS
   cx<float>* rs = reinterpret_cast<cx<float>*>(kap_t + TS);          // TS*mh*2 (x, y of r)
   bool use_r = a.resid != nullptr;
   Seam<float> sf = seam_load<float>(a.ph, a.K, k, n);
   Seam<HI> sh = seam_load<HI>(a.ph, a.K, k, n);
   // a launch accumulates the entries [ebase, ebase + MAXE*GT) of the lower
   // triangle (ns <= 48: one launch; larger blocks take several)
+  // Few entries (blocks of up to 21 columns alone): the threads split into
+  // ngr groups that take every ngr-th site of a tile and add up at the end
   constexpr int MAXE = 5;
-  cx<float> acc_a[MAXE], acc_m[MAXE];
+  const int ngr = nent < GT ? (GT / nent < TS ? GT / nent : TS) : 1, gr = ngr > 1 ? (int) threadIdx.x / nent : 0;
+  const int et = ngr > 1 ? (int) threadIdx.x - gr * nent : (int) threadIdx.x;
+  cx<float> acc_a[ALLHI ? 1 : MAXE], acc_m[ALLHI ? 1 : MAXE];
   cx<HI> hacc_a[MAXE], hacc_m[MAXE];
   int ei[MAXE], ej[MAXE];
+#pragma unroll
   for (int t = 0; t < MAXE; t++) {
-    acc_a[t] = czero<float>(); acc_m[t] = czero<float>();
+    if constexpr (!ALLHI) acc_a[t] = acc_m[t] = czero<float>();
     hacc_a[t] = czero<HI>(); hacc_m[t] = czero<HI>();
-    int e = ebase + threadIdx.x + t * GT;
+    int e = ebase + et + t * GT;
     ei[t] = -1; ej[t] = -1;
-    if (e < nent) {
+    if (e < nent && gr < ngr) {
       // row-major lower triangle: e = i(i+1)/2 + j, j <= i
       int i = (int) ((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
       while (i * (i + 1) / 2 > e) i--;
@@ -285,7 +323,7 @@ __global__ void k_block_gram(GramArgs a, int mh, int ebase) {
       ei[t] = i; ej[t] = e - i * (i + 1) / 2;
     }
   }
-  HI mmh = sget<HI>(a.sixth), fourh = rc<HI>(4.0f);
+  HI mmh = sget<HI>(a.sixth);
   float mmf = a.sixth.hi;
   size_t nsite = (size_t) n * n;
   size_t per = (nsite + a.chunks - 1) / a.chunks;
@@ -303,20 +341,22 @@ __global__ void k_block_gram(GramArgs a, int mh, int ebase) {
       cx<float>* ls = lo + ((size_t) ts * ns + col) * 5;
       if (col < mh) {
         cx<HI> c, x0, y0, mxv, myv;
-        if (prec == MX_CDD) {
-          EA<cdd, HI> E{(const cdd*) a.ptrs[b] + o0, n, m, sh};
+        // float-float blocks in float-float arithmetic, FP64 blocks in FP64
+        using SH = typename HiStore<HI>::T;
+        auto body = [&](const auto& E) {
           c = curlc<HI>(E, i, j); x0 = E(0, i, j); y0 = E(1, i, j);
-          mxv = scal(mmh, scal(fourh, x0) + E(0, i, j + 1) + E(0, i, j - 1));
-          myv = scal(mmh, scal(fourh, y0) + E(1, i + 1, j) + E(1, i - 1, j));
-        } else {
-          EA<double2, HI> E{(const double2*) a.ptrs[b] + o0, n, m, sh};
-          c = curlc<HI>(E, i, j); x0 = E(0, i, j); y0 = E(1, i, j);
-          mxv = scal(mmh, scal(fourh, x0) + E(0, i, j + 1) + E(0, i, j - 1));
-          myv = scal(mmh, scal(fourh, y0) + E(1, i + 1, j) + E(1, i - 1, j));
-        }
-        cx<HI>* hs = hi + ((size_t) ts * mh + col) * 5;
+          mxv = scal(mmh, times4(x0) + E(0, i, j + 1) + E(0, i, j - 1));
+          myv = scal(mmh, times4(y0) + E(1, i + 1, j) + E(1, i - 1, j));
+        };
+        const SH* eb = (const SH*) a.ptrs[b] + o0;
+        if (i > 0 && i < n - 1 && j > 0 && j < n - 1) body(EAI<SH, HI>{eb, n, m});
+        else body(EA<SH, HI>{eb, n, m, sh});
+        cx<HI>* hs = hi + ((size_t) ts * mh + col) * 6;
         hs[0] = c; hs[1] = x0; hs[2] = y0; hs[3] = mxv; hs[4] = myv;
-        ls[0] = to_cf(c); ls[1] = to_cf(x0); ls[2] = to_cf(y0); ls[3] = to_cf(mxv); ls[4] = to_cf(myv);
+        hs[5] = scal(KapHi<HI>::get(a.kap, site), c);
+        if constexpr (!ALLHI) {   // (rounded for entries with a c64 column)
+          ls[0] = to_cf(c); ls[1] = to_cf(x0); ls[2] = to_cf(y0); ls[3] = to_cf(mxv); ls[4] = to_cf(myv);
+        }
       } else {
         const void* pb = a.ptrs[b];
         auto X = [&](int p, int ii, int jj) {
@@ -345,33 +385,29 @@ __global__ void k_block_gram(GramArgs a, int mh, int ebase) {
       }
     for (int ts = threadIdx.x; ts < TS; ts += GT) {
       size_t site = base + ts;
-      if (site < s1) {
-        kap_t[ts] = a.kap.f[site];
-        kap_h[ts] = KapHi<HI>::get(a.kap, site);
-      } else {
-        kap_t[ts] = 0.0f;
-        kap_h[ts] = Real<HI>::zero();
-      }
+      kap_t[ts] = site < s1 ? a.kap.f[site] : 0.0f;
     }
     __syncthreads();
     int nts = (int) (s1 - base < (size_t) TS ? s1 - base : (size_t) TS);
+#pragma unroll
     for (int t = 0; t < MAXE; t++) {
       int i = ei[t], j = ej[t];
       if (i < 0) continue;
-      if (i < mh && j < mh) {
+      if (ALLHI || (i < mh && j < mh)) {
         cx<HI> sa = czero<HI>(), sm2 = czero<HI>();
-        for (int ts = 0; ts < nts; ts++) {
-          const cx<HI>* hs = hi + (size_t) ts * mh * 5;
-          sa += scal(kap_h[ts], conjc(hs[i * 5]) * hs[j * 5]);
-          sm2 += conjc(hs[i * 5 + 1]) * hs[j * 5 + 3] + conjc(hs[i * 5 + 2]) * hs[j * 5 + 4];
+        for (int ts = gr; ts < nts; ts += ngr) {
+          const cx<HI>* hs = hi + (size_t) ts * mh * 6;
+          gram_mac(sa, hs[i * 6], hs[j * 6 + 5]);
+          gram_mac(sm2, hs[i * 6 + 1], hs[j * 6 + 3]);
+          gram_mac(sm2, hs[i * 6 + 2], hs[j * 6 + 4]);
         }
         hacc_a[t] += sa;
         hacc_m[t] += sm2;
-      } else if (use_r && j < mh) {
+      } else if constexpr (!ALLHI) if (use_r && j < mh) {
         // cross entry s_i^H (A+M) e_j = theta_j s_i^H M e_j + s_i^H r_j: only
         // s_i^H r_j is accumulated here, the rest is added at the end
         cx<float> sa = czero<float>(), sm2 = czero<float>();
-        for (int ts = 0; ts < nts; ts++) {
+        for (int ts = gr; ts < nts; ts += ngr) {
           const cx<float>* ls = lo + (size_t) ts * ns * 5;
           const cx<float>* rr = rs + (size_t) ts * mh * 2;
           sa += conjc(ls[i * 5 + 1]) * rr[j * 2] + conjc(ls[i * 5 + 2]) * rr[j * 2 + 1];
@@ -381,7 +417,7 @@ __global__ void k_block_gram(GramArgs a, int mh, int ebase) {
         acc_m[t] += sm2;
       } else {
         cx<float> sa = czero<float>(), sm2 = czero<float>();
-        for (int ts = 0; ts < nts; ts++) {
+        for (int ts = gr; ts < nts; ts += ngr) {
           const cx<float>* ls = lo + (size_t) ts * ns * 5;
           sa += scal(kap_t[ts], conjc(ls[i * 5]) * ls[j * 5]);
           sm2 += conjc(ls[i * 5 + 1]) * ls[j * 5 + 3] + conjc(ls[i * 5 + 2]) * ls[j * 5 + 4];
@@ -393,25 +429,34 @@ __global__ void k_block_gram(GramArgs a, int mh, int ebase) {
   }
   double axy = (double) n * (double) n;
   double* out = a.partial + (((size_t) k * a.chunks + chunk) * nent) * 4;
+  double* red = smd;   // [ngr][nent][4], over the staging
+  if (ngr > 1) __syncthreads();
+#pragma unroll
   for (int t = 0; t < MAXE; t++) {
-    int e = ebase + threadIdx.x + t * GT;
-    if (e >= nent) continue;
-    double ar = Real<HI>::to_double(hacc_a[t].re) + (double) acc_a[t].re;
-    double ai = Real<HI>::to_double(hacc_a[t].im) + (double) acc_a[t].im;
-    double mr = Real<HI>::to_double(hacc_m[t].re) + (double) acc_m[t].re;
-    double mi = Real<HI>::to_double(hacc_m[t].im) + (double) acc_m[t].im;
-    // A + M = axy * (sum over cells of kappa conj(curl_i) curl_j) + M, or
-    // for the residual form of the cross entries theta_j * M + s_i^H r_j
-    if (use_r && ei[t] >= mh && ej[t] < mh) {
-      double th = a.theta[(size_t) k * m + ej[t]];
-      out[(size_t) e * 4 + 0] = th * mr + ar;
-      out[(size_t) e * 4 + 1] = th * mi + ai;
-    } else {
-      out[(size_t) e * 4 + 0] = axy * ar + mr;
-      out[(size_t) e * 4 + 1] = axy * ai + mi;
+    int e = ebase + et + t * GT;
+    if (ei[t] < 0) continue;
+    double q[4] = {Real<HI>::to_double(hacc_a[t].re), Real<HI>::to_double(hacc_a[t].im),
+                   Real<HI>::to_double(hacc_m[t].re), Real<HI>::to_double(hacc_m[t].im)};
+    if constexpr (!ALLHI) {
+      q[0] += (double) acc_a[t].re; q[1] += (double) acc_a[t].im;
+      q[2] += (double) acc_m[t].re; q[3] += (double) acc_m[t].im;
     }
-    out[(size_t) e * 4 + 2] = mr;
-    out[(size_t) e * 4 + 3] = mi;
+    if (ngr > 1) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) red[((size_t) gr * nent + e) * 4 + c] = q[c];
+      continue;
+    }
+    gram_entry(a, k, e, ei[t], ej[t], mh, use_r, axy, q, out);
+  }
+  if (ngr > 1) {
+    __syncthreads();
+    if (gr == 0) {
+      double q[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int g = 0; g < ngr; g++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) q[c] += red[((size_t) g * nent + et) * 4 + c];
+      gram_entry(a, k, et, ei[0], ej[0], mh, use_r, axy, q, out);
+    }
   }
 }
 
@@ -475,7 +520,11 @@ template <> struct CoefGet<double> {
   }
 };
 
-template <typename SO, typename RO>
+// HIDD: the blocks that are not c64 are float-float (else FP64).  A run-time
+// choice made FP64 blocks pay for the other storage's conversions, which
+// occupy the FP64 pipe even where no lane takes them: 120^2 x 11 vectors x 5
+// k-points 0.41 -> 0.21 ms.
+template <typename SO, typename RO, bool HIDD>
 __global__ void k_block_combine(CombArgs a, SO* __restrict__ out) {
   // block (m, rows): x = output column, y = entry (plane, site); grid.y = k.
   // The coefficients are staged once per block in shared memory in the
@@ -507,9 +556,11 @@ __global__ void k_block_combine(CombArgs a, SO* __restrict__ out) {
   size_t kbase = (size_t) k * per_k + (size_t) ent * m;
   cx<RO> acc_hi = czero<RO>();
   cx<float> acc_lo = czero<float>();
+  bool any_lo = false;
   for (int b = 0; b < a.nb; b++) {
     int prec = a.precs[b];
     if (prec == MX_C64) {
+      any_lo = true;
       const float2* src = (const float2*) a.ptrs[b] + kbase;
       const cx<float>* cc = clo + j * nsrc + b * m;
       for (int i = 0; i < m; i++) {
@@ -519,13 +570,15 @@ __global__ void k_block_combine(CombArgs a, SO* __restrict__ out) {
     } else {
       const cx<RO>* cc = chi + j * nsrc + b * m;
       for (int i = 0; i < m; i++) {
-        cx<RO> v = prec == MX_CDD ? Store<cdd, RO>::ld((const cdd*) a.ptrs[b] + kbase + i)
-                                  : Store<double2, RO>::ld((const double2*) a.ptrs[b] + kbase + i);
+        cx<RO> v;
+        if constexpr (HIDD) v = Store<cdd, RO>::ld((const cdd*) a.ptrs[b] + kbase + i);
+        else v = Store<double2, RO>::ld((const double2*) a.ptrs[b] + kbase + i);
         acc_hi += cc[i] * v;
       }
     }
   }
-  cx<RO> res = acc_hi + mkc(Real<RO>::from_float(acc_lo.re), Real<RO>::from_float(acc_lo.im));
+  cx<RO> res = acc_hi;
+  if (any_lo) res += mkc(Real<RO>::from_float(acc_lo.re), Real<RO>::from_float(acc_lo.im));
   Store<SO, RO>::st(out + kbase + j, res);
 }
 
@@ -1094,8 +1147,9 @@ extern "C" int mxk_block_gram(int n, int m, int K, const double* ph, mxk_kappa k
   int mh = all128 ? a.ns : (precs[0] == MX_C64 ? 0 : m);
   size_t hsz = hi_dd ? sizeof(cx<dd>) : sizeof(cx<double>);
   if (resid && (all128 || mh == 0)) return (int) cudaErrorInvalidValue;
-  size_t smem = hsz * TS * mh * 5 + sizeof(cx<float>) * TS * a.ns * 5 + (hsz / 2 + sizeof(float)) * TS
+  size_t smem = hsz * TS * mh * 6 + (all128 ? 0 : sizeof(cx<float>) * TS * a.ns * 5) + sizeof(float) * TS
                 + sizeof(cx<float>) * TS * mh * 2 + 16;
+  if (smem < (size_t) GT * 4 * sizeof(double)) smem = (size_t) GT * 4 * sizeof(double);   // the groups' sums
   bool lo_rest = true;
   for (int q = 1; q < nb; q++) lo_rest = lo_rest && precs[q] == MX_C64;
   if (hi_dd && lo_rest && m <= 16 && nb <= 3 && (nb == 1 || resid)) {
@@ -1103,11 +1157,14 @@ extern "C" int mxk_block_gram(int n, int m, int K, const double* ph, mxk_kappa k
     cudaFuncSetAttribute(k_block_gram_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
     k_block_gram_split<<<dim3(a.chunks, K, nb > 1 ? 2 : 1), GS_T, sm, st>>>(a);
   } else if (hi_dd) {
-    cudaFuncSetAttribute(k_block_gram<dd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<dd><<<g, GT, smem, st>>>(a, mh, eb);
+    cudaFuncSetAttribute(k_block_gram<dd, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<dd, false><<<g, GT, smem, st>>>(a, mh, eb);
+  } else if (all128) {
+    cudaFuncSetAttribute(k_block_gram<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, true><<<g, GT, smem, st>>>(a, mh, eb);
   } else {
-    cudaFuncSetAttribute(k_block_gram<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double><<<g, GT, smem, st>>>(a, mh, eb);
+    cudaFuncSetAttribute(k_block_gram<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, false><<<g, GT, smem, st>>>(a, mh, eb);
   }
   MX_CHECK_LAUNCH();
   size_t work = (size_t) nent * K;
@@ -1159,24 +1216,26 @@ extern "C" int mxk_block_combine(int n, int m, int K, int nb, const int* precs, 
     return 0;
   }
   if (m > 256) return (int) cudaErrorInvalidValue;
+  for (int q = 0; q < nb; q++)   // one storage for all blocks that are not c64
+    for (int r = 0; r < q; r++)
+      if (precs[q] != precs[r] && precs[q] != MX_C64 && precs[r] != MX_C64) return (int) cudaErrorInvalidValue;
   unsigned rows = 256 / m;
   dim3 g((unsigned) ((2 * (size_t) n * n + rows - 1) / rows), K), b(m, rows);
   size_t ncoef = (size_t) nb * m * m;
   // the coefficients staged per block exceed the default 48 KB for blocks
   // of more than about 24 vectors
-  if (pout == MX_CDD) {
-    size_t sm = ncoef * (sizeof(cx<dd>) + sizeof(cx<float>));
-    cudaFuncSetAttribute(k_block_combine<cdd, dd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
-    k_block_combine<cdd, dd><<<g, b, sm, st>>>(a, (cdd*) out);
-  } else if (pout == MX_C128) {
-    size_t sm = ncoef * (sizeof(cx<double>) + sizeof(cx<float>));
-    cudaFuncSetAttribute(k_block_combine<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
-    k_block_combine<double2, double><<<g, b, sm, st>>>(a, (double2*) out);
-  } else {
-    size_t sm = ncoef * (sizeof(cx<float>) * 2);
-    cudaFuncSetAttribute(k_block_combine<float2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
-    k_block_combine<float2, float><<<g, b, sm, st>>>(a, (float2*) out);
-  }
+  bool hidd = false;
+  for (int q = 0; q < nb; q++) hidd = hidd || precs[q] == MX_CDD;
+#define MX_CB(SO, RO, DD)                                                                                             \
+  do {                                                                                                                \
+    const size_t sm = ncoef * (sizeof(cx<RO>) + sizeof(cx<float>));                                                   \
+    cudaFuncSetAttribute(k_block_combine<SO, RO, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);          \
+    k_block_combine<SO, RO, DD><<<g, b, sm, st>>>(a, (SO*) out);                                                      \
+  } while (0)
+  if (pout == MX_CDD) { if (hidd) MX_CB(cdd, dd, true); else MX_CB(cdd, dd, false); }
+  else if (pout == MX_C128) { if (hidd) MX_CB(double2, double, true); else MX_CB(double2, double, false); }
+  else { if (hidd) MX_CB(float2, float, true); else MX_CB(float2, float, false); }
+#undef MX_CB
   MX_CHECK_LAUNCH();
   return 0;
 }

@@ -135,3 +135,32 @@ def test_sensitivity_shares(oracle, n, K, m):
     got = mx.eps_sensitivity(n, kap, fac, vec, w)
     want = sum(oracle.eps_sensitivity(n, kap, *fac[k], vec[k], w[k]) for k in range(K))
     assert rel(got, want) < 1e-12
+
+
+@pytest.mark.parametrize("n, m, K", [(6, 1, 2), (10, 4, 1), (22, 11, 2), (16, 21, 1), (12, 32, 1)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+def test_gram_and_combination_block_sizes(n, m, K, prec):
+    """Ritz products and combinations of one block, whose entries leave the
+    products' threads in 16, several or one group(s) and several entries a
+    thread, against matrices put together from the dense operator."""
+    rng = np.random.default_rng(m)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    g = mx.Grid(n, K, kap, FACTORS[:K])
+    x = mx.Edge(g, m, prec, cv(rng, K, m, 2 * n * n))
+    u = x.get()
+    Kd, Md = mx.Matrix(2 * n * n, K), mx.Matrix(2 * n * n, K)
+    mx.check(mx.lib().densematrix_edge2d_gpu(mx.fz(1.0), mx.fz(1.0), g.h, Kd.h))
+    mx.check(mx.lib().densematrix_edge2d_gpu(mx.fz(0.0), mx.fz(1.0), g.h, Md.h))
+    Kd, Md = Kd.get(), Md.get()
+    a, b = np.zeros((K, m, m), complex), np.zeros((K, m, m), complex)
+    mx.check(mx.lib().gram_edge2d_gpu(x.h, mx._ptr(a), mx._ptr(b)))
+    tol = {mx.C128: 1e-13, mx.CDD: 1e-12, mx.C64: 2e-6}[prec]
+    for k in range(K):
+        assert rel(a[k].T, u[k].conj() @ Kd[k] @ u[k].T) < tol
+        assert rel(b[k].T, u[k].conj() @ Md[k] @ u[k].T) < tol
+    coef, y = cv(rng, K, m, m), mx.Edge(g, m, prec)
+    ct = np.ascontiguousarray(coef.transpose(0, 2, 1))
+    mx.check(mx.lib().lincomb_edge2d_gpu(mx._ptr(ct), x.h, y.h))
+    got = y.get()
+    for k in range(K):
+        assert rel(got[k], coef[k].T @ u[k]) < {mx.C128: 1e-14, mx.CDD: 1e-13, mx.C64: 2e-6}[prec] * m
