@@ -375,8 +375,9 @@ int mxg_solver_check_fp64(mxg_solver *s, double *res);
  * missed the tolerance and were solved again from a cold start */
 int mxg_solver_restarts(const mxg_solver *s);
 /* CUDA-event timing, on the solver's stream, of three launch sequences at
- * the finest level: node Gauss-Seidel sweeps of the gradient lifting
- * (MXG_KT_NODE_GS), AFW sweeps of the preconditioner (MXG_KT_AFW) and the
+ * the finest level: the smoothing launches of the gradient lifting's node
+ * V-cycles (MXG_KT_NODE_GS: sweeps, or sweeps with the residual, restriction
+ * or prolongation they are fused with), AFW sweeps of the preconditioner (MXG_KT_AFW) and the
  * Gram matrices of the Ritz step (MXG_KT_GRAM).  With profiling enabled the
  * solver launches the V-cycles directly (no CUDA graph) so that every sweep
  * carries its own events.  kernel_time returns, since profiling was enabled,

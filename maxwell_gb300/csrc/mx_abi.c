@@ -45,6 +45,7 @@ struct node2d_gpu {
   const grid2d_gpu *gr;
   int m, prec;
   void *d;
+  void *work;          /* a vector of scratch that vcycle_node2d_gpu keeps with its x[L] */
 };
 
 struct matrix_gpu {
@@ -492,11 +493,11 @@ int hcycle_edge2d_gpu(int L, int nu, const matrix_gpu *Ac, edge2d_gpu **b, edge2
     if(b[l]->prec != d[l]->prec) return MXG_EINVAL;
     TRY(mxk_edge_apply(g->n, x[l]->m, g->K, g->ph, kap_of(g), -1.0, -1.0, 0, 1.0, x[l]->prec, x[l]->d,
                        d[l]->prec, b[l]->d, d[l]->d, g->st));
-    TRY(mxk_adjgradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, 0.0, d[l]->prec, d[l]->d, bg[l]->prec, bg[l]->d, g->st));
+    TRY(mxk_adjgradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, 0.0, 0, d[l]->prec, d[l]->d, bg[l]->prec, bg[l]->d, g->st));
     TRY(zero_node2d_gpu(xg[l]));
     for(i = 0; i < nu; i++)
       TRY(mxk_node_gs(g->n, x[l]->m, g->K, g->ph, 1.0, 0, xg[l]->prec, bg[l]->d, xg[l]->d, g->st));
-    TRY(mxk_gradient(g->n, x[l]->m, g->K, g->ph, 1.0, xg[l]->prec, xg[l]->d, x[l]->prec, x[l]->d, g->st));
+    TRY(mxk_gradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, xg[l]->prec, xg[l]->d, x[l]->prec, x[l]->d, g->st));
     TRY(mxk_edge_apply(g->n, x[l]->m, g->K, g->ph, kap_of(g), -1.0, -1.0, 0, 1.0, x[l]->prec, x[l]->d,
                        d[l]->prec, b[l]->d, d[l]->d, g->st));
     TRY(zero_edge2d_gpu(b[l - 1]));
@@ -516,11 +517,11 @@ int hcycle_edge2d_gpu(int L, int nu, const matrix_gpu *Ac, edge2d_gpu **b, edge2
     TRY(mxk_edge_prolong(g->n / 2, x[l]->m, g->K, g->ph, 1.0, x[l]->prec, x[l - 1]->d, x[l]->d, g->st));
     TRY(mxk_edge_apply(g->n, x[l]->m, g->K, g->ph, kap_of(g), -1.0, -1.0, 0, 1.0, x[l]->prec, x[l]->d,
                        d[l]->prec, b[l]->d, d[l]->d, g->st));
-    TRY(mxk_adjgradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, 0.0, d[l]->prec, d[l]->d, bg[l]->prec, bg[l]->d, g->st));
+    TRY(mxk_adjgradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, 0.0, 0, d[l]->prec, d[l]->d, bg[l]->prec, bg[l]->d, g->st));
     TRY(zero_node2d_gpu(xg[l]));
     for(i = 0; i < nu; i++)
       TRY(mxk_node_gs(g->n, x[l]->m, g->K, g->ph, 1.0, 1, xg[l]->prec, bg[l]->d, xg[l]->d, g->st));
-    TRY(mxk_gradient(g->n, x[l]->m, g->K, g->ph, 1.0, xg[l]->prec, xg[l]->d, x[l]->prec, x[l]->d, g->st));
+    TRY(mxk_gradient(g->n, x[l]->m, g->K, g->ph, 1.0, 0, xg[l]->prec, xg[l]->d, x[l]->prec, x[l]->d, g->st));
     for(i = 0; i < nu; i++)
       TRY(gs_simple(1.0, 1.0, b[l], x[l], 1));
   }
@@ -567,6 +568,7 @@ void del_node2d_gpu(node2d_gpu *x)
 {
   if(!x) return;
   cudaFree(x->d);
+  cudaFree(x->work);
   free(x);
 }
 
@@ -631,14 +633,14 @@ int gradient_node2d_gpu(mxg_field alpha, const node2d_gpu *x, edge2d_gpu *y)
 {
   const grid2d_gpu *g = x->gr;
   if(x->m != y->m || g->n != y->gr->n) return MXG_EINVAL;
-  return mxk_gradient(g->n, x->m, g->K, g->ph, creal_(alpha), x->prec, x->d, y->prec, y->d, g->st);
+  return mxk_gradient(g->n, x->m, g->K, g->ph, creal_(alpha), 0, x->prec, x->d, y->prec, y->d, g->st);
 }
 
 int adjgradient_node2d_gpu(mxg_field alpha, const edge2d_gpu *x, node2d_gpu *y)
 {
   const grid2d_gpu *g = x->gr;
   if(x->m != y->m || g->n != y->gr->n) return MXG_EINVAL;
-  return mxk_adjgradient(g->n, x->m, g->K, g->ph, creal_(alpha), 0, 1.0, x->prec, x->d, y->prec, y->d, g->st);
+  return mxk_adjgradient(g->n, x->m, g->K, g->ph, creal_(alpha), 0, 1.0, 0, x->prec, x->d, y->prec, y->d, g->st);
 }
 
 /* The level from which vcycle_node2d_gpu runs in one launch (0: none): a
@@ -670,9 +672,53 @@ static int gs_cycle(const node2d_gpu *b, node2d_gpu *x, int dir)
   return mxk_node_gs(g->n, x->m, g->K, g->ph, 1.0, dir, x->prec, b->d, x->d, g->st);
 }
 
+/* The fine levels of vcycle_node2d_gpu on planar vectors (the levels up to lc
+ * in one launch): every level above lc has a band kernel, the same factors and
+ * shapes, and there is memory for a planar copy of b[L], kept with x[L]. */
+static int planar_cycle_ok(int L, int lc, int nu, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
+{
+  const grid2d_gpu *g0 = x[0]->gr;
+  int l;
+  if(lc == 0 || lc == L || mxk_node_gs_oop_ok(x[L]->gr->n, x[L]->m, x[L]->prec)) return 0;
+  for(l = lc + 1; l <= L; l++) {
+    const grid2d_gpu *g = x[l]->gr;
+    if(!mxk_node_band_ok(g->n, x[l]->m, nu, x[l]->prec) || g->n != g0->n << l || g->K != g0->K
+       || memcmp(g->h_ph, g0->h_ph, sizeof(double) * 4 * g0->K) || x[l]->m != x[0]->m || x[l]->prec != x[0]->prec
+       || b[l]->m != x[0]->m || b[l]->prec != x[0]->prec || b[l]->gr->n != g->n || b[l]->gr->K != g->K
+       || d[l]->m != x[0]->m || d[l]->prec != x[0]->prec || d[l]->gr->n != g->n || d[l]->gr->K != g->K
+       || b[l]->d == x[l]->d || b[l]->d == d[l]->d || x[l]->d == d[l]->d)
+      return 0;
+  }
+  if(!x[L]->work && cudaMalloc(&x[L]->work, nlen(x[L]) * mxk_elem_size(x[L]->prec))) {
+    cudaGetLastError();
+    x[L]->work = 0;
+    return 0;
+  }
+  return 1;
+}
+
+static int planar_cycle(int L, int lc, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
+{
+  const grid2d_gpu *g = x[L]->gr;
+  int l, m = x[L]->m, K = g->K;
+  /* b[L] into the scratch vector, x[L] into d[L]; level L goes d -> x -> d */
+  TRY(mxk_node_planar(g->n, m, K, 1, b[L]->d, x[L]->work, g->st));
+  TRY(mxk_node_planar(g->n, m, K, 1, x[L]->d, d[L]->d, g->st));
+  TRY(mxk_node_band_pre(g->n, m, K, nu, g->ph, x[L]->work, d[L]->d, x[L]->d, b[L - 1]->d, g->st));
+  for(l = L - 1; l > lc; l--)
+    TRY(mxk_node_band_pre(x[l]->gr->n, m, K, nu, g->ph, b[l]->d, 0, d[l]->d, b[l - 1]->d, g->st));
+  TRY(mxk_node_vcycle(x[0]->gr->n, lc, m, K, nu, 1, 1, 1, g->ph, Ac->d, 0, x[lc]->prec, b[lc]->d, x[lc]->d, g->st));
+  for(l = lc + 1; l < L; l++)
+    TRY(mxk_node_band_post(x[l]->gr->n, m, K, nu, g->ph, b[l]->d, d[l]->d, x[l - 1]->d, x[l]->d, g->st));
+  TRY(mxk_node_band_post(g->n, m, K, nu, g->ph, x[L]->work, x[L]->d, x[L - 1]->d, d[L]->d, g->st));
+  TRY(mxk_node_planar(g->n, m, K, 0, d[L]->d, x[L]->d, g->st));
+  return (int) cudaStreamSynchronize(g->st);
+}
+
 int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
 {
   int l, i, lc = fused_level_n(L, Ac, b, x);
+  if(planar_cycle_ok(L, lc, nu, b, x, d)) return planar_cycle(L, lc, nu, Ac, b, x, d);
   for(l = L; l > lc; l--) {
     const grid2d_gpu *g = x[l]->gr;
     for(i = 0; i < nu; i++)
@@ -685,7 +731,7 @@ int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2
   }
   if(lc > 0) {
     const grid2d_gpu *g = x[lc]->gr;
-    TRY(mxk_node_vcycle(x[0]->gr->n, lc, x[lc]->m, g->K, nu, 1, lc < L, g->ph, Ac->d, 0, x[lc]->prec, b[lc]->d,
+    TRY(mxk_node_vcycle(x[0]->gr->n, lc, x[lc]->m, g->K, nu, 1, lc < L, 0, g->ph, Ac->d, 0, x[lc]->prec, b[lc]->d,
                         x[lc]->d, g->st));
   }
   else if(Ac) {

@@ -108,18 +108,30 @@ int mxk_node_rr_get_strips(void);
  * level, x starting from zero where zero is set.  mxk_node_vcycle_top: the
  * highest level up to `top` that this form takes (0: none) */
 int mxk_node_vcycle_top(int n0, int top, int prec);
-int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, const double *phases,
-                    const double *ainv, const void *ainv_c64, int prec, const void *b, void *x, mx_stream s);
+int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
+                    const double *phases, const double *ainv, const void *ainv_c64, int prec,
+                    const void *b, void *x, mx_stream s);
+/* one level's two sides of a V-cycle on planar c64 vectors ([k][v][j][i]),
+ * xin (NULL: zero) and xout distinct: nu forward sweeps and the restricted
+ * residual bc; the prolongation of xc and nu backward sweeps */
+int mxk_node_band_ok(int n, int m, int nu, int prec);
+int mxk_node_band_pre(int n, int m, int K, int nu, const double *phases, const void *b, const void *xin,
+                      void *xout, void *bc, mx_stream s);
+int mxk_node_band_post(int n, int m, int K, int nu, const double *phases, const void *b, const void *xin,
+                       const void *xc, void *xout, mx_stream s);
+/* c64 node vectors [k][j][i][v] -> planar (to = 1) or back (to = 0) */
+int mxk_node_planar(int n, int m, int K, int to, const void *src, void *dst, mx_stream s);
 int mxk_node_prolong(int nc, int m, int K, const double *phases, double alpha,
                      int prec, const void *c, void *f, mx_stream s);
 int mxk_node_restrict(int nc, int m, int K, const double *phases, double alpha,
                       int prec, const void *f, void *c, mx_stream s);
-/* e = ce*e + alpha * G v  (node -> edge) */
-int mxk_gradient(int n, int m, int K, const double *phases, double alpha,
+/* e = ce*e + alpha * G v  (node -> edge); planar: v is a planar c64 vector */
+int mxk_gradient(int n, int m, int K, const double *phases, double alpha, int planar,
                  int prec_v, const void *v, int prec_e, void *e, mx_stream s);
-/* v = cv*v + alpha * G^H (mass ? M e : e)  (edge -> node) */
+/* v = cv*v + alpha * G^H (mass ? M e : e)  (edge -> node); planar (c64, cv = 0):
+ * v is written as a planar vector */
 int mxk_adjgradient(int n, int m, int K, const double *phases, double alpha, int mass,
-                    double cv, int prec_e, const void *e, int prec_v, void *v, mx_stream s);
+                    double cv, int planar, int prec_e, const void *e, int prec_v, void *v, mx_stream s);
 
 /* ---- block BLAS-1 (len complex entries) ---- */
 int mxk_zero(int prec, void *x, size_t len, mx_stream s);

@@ -332,9 +332,9 @@ static int run(int n, int K, int m, int reps, mxg_kbench_row *rows, int maxrows,
     TIME("node_prolong_c64", (V8 / 4 + 2 * V8) * s8, 1,
          mxk_node_prolong(n / 2, m, K, ph, 1.0, MX_C64, nbc, nx, st));
     TIME("adjgradient_mass_cdd_to_c64", E8 * s16 + V8 * s8, 1,
-         mxk_adjgradient(n, m, K, ph, 1.0, 1, 0.0, MX_CDD, E, MX_C64, nb, st));
+         mxk_adjgradient(n, m, K, ph, 1.0, 1, 0.0, 0, MX_CDD, E, MX_C64, nb, st));
     TIME("gradient_c64_to_cdd", V8 * s8 + 2 * E8 * s16, 1,
-         mxk_gradient(n, m, K, ph, -1e-3, MX_C64, nx, MX_CDD, E, st));
+         mxk_gradient(n, m, K, ph, -1e-3, 0, MX_C64, nx, MX_CDD, E, st));
     TIME("block_residual_cdd", E8 * s16 + E8 * s8 + 8.0 * nn, 1,
          (cudaMemsetAsync(stats, 0, sizeof(double) * 5 * m * K, st),
           mxk_block_residual(n, m, K, ph, kap, mu, MX_CDD, E, MX_C64, r, stats, st)));

@@ -247,7 +247,7 @@ __device__ void coarse_solve(int N, const MS* __restrict__ ainv, cx<R>* X, const
 
 template <typename S, typename R, typename MS>
 __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero,
-                                                   const double* __restrict__ ph, Sc third,
+                                                   int planar, const double* __restrict__ ph, Sc third,
                                                    const MS* __restrict__ ainv, const S* __restrict__ b, S* x) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const int v = blockIdx.x % m, k = blockIdx.x / m, n = n0 << top, nn = n * n;
@@ -260,11 +260,13 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
     return p;
   };
   const Seam<R> sm0 = seam_load<R>(ph, K, k, n);
-  const S* bk = b + (size_t) k * nn * m + v;
-  S* xk = x + (size_t) k * nn * m + v;
+  // element e of vector v: [k][e][v], or [k][v][e] where planar
+  const size_t at0 = (size_t) k * nn * m + (planar ? (size_t) v * nn : (size_t) v), es = planar ? 1 : m;
+  const S* bk = b + at0;
+  S* xk = x + at0;
   for (int e = threadIdx.x; e < nn; e += NCT) {
-    X[nn + e] = Store<S, R>::ld(bk + (size_t) e * m);
-    X[e] = zero ? czero<R>() : Store<S, R>::ld(xk + (size_t) e * m);
+    X[nn + e] = Store<S, R>::ld(bk + e * es);
+    X[e] = zero ? czero<R>() : Store<S, R>::ld(xk + e * es);
   }
   __syncthreads();
   for (int c = 0; c < cycles; c++) {
@@ -291,7 +293,410 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
       smooth<R>(nl, nu, 1, Xl, Xl + nl * nl, sm);
     }
   }
-  for (int e = threadIdx.x; e < nn; e += NCT) Store<S, R>::st(xk + (size_t) e * m, X[e]);
+  for (int e = threadIdx.x; e < nn; e += NCT) Store<S, R>::st(xk + e * es, X[e]);
+}
+
+// ------------------------------------------------------------------
+// The fine levels: all that a V-cycle does with a level on one side of the
+// coarse correction in one pass over memory, for c64 vectors stored one after
+// the other ([k][v][j][i], planar).
+//   PRE   x' = nu forward sweeps on x (or zero) and b, and the restriction of
+//         b - L x' (node2d.c:1352-1389's first half of a level)
+//   POST  x' = nu backward sweeps on x + P xc and b
+// A CTA takes a band of B rows of one vector, with the rows around it that
+// the band's final values depend on: a phase (half a sweep) uses up one row on
+// each side, the residual and its restriction one and two more.  Row 0 is
+// swept before the odd rows and row n-1 after the even ones, which lets a
+// dependence run two rows in one phase across the seam; bands start at row 0
+// or 8 and more, and end at row n or n - 8 and less, where the same halo
+// holds.  The result goes to another vector, since neighbour bands read the
+// old one.  Rows beyond the seam are loaded with their phase, so only the
+// columns wrap.  x sits in shared memory (two CTAs per SM), b comes through L2
+// for every sweep.  A warp sweeps a row in segments of 128 columns, four per
+// lane: run of four, shuffle scan of the runs with factor 8^-4, carry from the
+// segment before.
+//
+// Traffic per side: x and b read with B + 11 (PRE) or B + 8 rows for B, x
+// written once, against 2 nu + .. passes of the separate kernels (a sweep 4
+// arrays, residual and restriction 2.25).  Bound by issue and the barriers of
+// the phases (53 % of issue slots, 0.84 GB of DRAM traffic per PRE call at
+// 512^2).  8 k-points x 16 vectors, nu = 2: PRE 0.455 ms at 512^2 against 0.69
+// for two sweeps and residual with restriction, 0.115 against 0.25 at 256^2;
+// POST 0.355 against 0.56 for prolongation and two sweeps.
+// ------------------------------------------------------------------
+constexpr int NBT = 512;
+
+__device__ __forceinline__ cx<float> dn_c(cx<float> v, int d) {
+  return mkc(__shfl_down_sync(0xffffffffu, v.re, d), __shfl_down_sync(0xffffffffu, v.im, d));
+}
+__device__ __forceinline__ cx<float> at_c(cx<float> v, int src) {
+  return mkc(__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src));
+}
+struct Two {
+  cx<float> a, b;   // columns c, c + 1
+};
+__device__ __forceinline__ Two ld2(const float2* p) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  return Two{mkc(v.x, v.y), mkc(v.z, v.w)};
+}
+__device__ __forceinline__ void st2(float2* p, Two t) {
+  *reinterpret_cast<float4*>(p) = make_float4(t.a.re, t.a.im, t.b.re, t.b.im);
+}
+__device__ __forceinline__ cx<float> ld1(const float2* p) { return mkc(p->x, p->y); }
+
+// A row in shared memory: segments of 128 columns, the column pairs 4l, 4l+1
+// of the lanes first, then the pairs 4l+2, 4l+3, so that a lane's four columns
+// are two conflict-free 16-byte accesses.
+__device__ __forceinline__ int pcol(int c) { return (c & ~127) + ((c & 2) << 5) + ((c & 124) >> 1) + (c & 1); }
+struct Four {
+  cx<float> v[4];
+};
+__device__ __forceinline__ Four ld4(const float2* p, int second) {
+  const Two a = ld2(p), b = ld2(p + second);
+  return Four{{a.a, a.b, b.a, b.b}};
+}
+__device__ __forceinline__ void st4(float2* p, int second, const Four& t) {
+  st2(p, Two{t.v[0], t.v[1]});
+  st2(p + second, Two{t.v[2], t.v[3]});
+}
+__device__ __forceinline__ cx<float> pick(bool c, cx<float> a, cx<float> b) { return mkc(c ? a.re : b.re, c ? a.im : b.im); }
+// 8^-4d, the carry's weight in lane d of a segment (below FP32's rounding past 3)
+__device__ __forceinline__ float pow84(int d) { return d < 4 ? __int_as_float((127 - 12 * d) << 23) : 0.0f; }
+
+// one row of one sweep by a warp; Xm, Xc, Xp: rows j-1, j, j+1 in shared
+// memory, bp: the phase of b's row where phased
+template <bool BACK>
+__device__ __forceinline__ void band_row(int n, const float2* Xm, float2* Xc, const float2* Xp,
+                                         const float2* __restrict__ B, bool phased, cx<float> bp, cx<float> xf) {
+  const int lane = threadIdx.x & 31, nseg = (n + 127) / 128, pl = pcol(n - 1);
+  const cx<float> xfc = conjc(xf);
+  // the sums of rows j-1 and j+1 in the columns across the seam, and the
+  // row's old value there that starts the recurrence
+  const cx<float> wl = xfc * (ld1(Xm + pl) + ld1(Xp + pl)), wr = xf * (ld1(Xm) + ld1(Xp));
+  const cx<float> old = BACK ? xf * ld1(Xc) : xfc * ld1(Xc + pl);
+  cx<float> carry = czero<float>(), first = czero<float>();
+#pragma unroll 1
+  for (int q = 0; q < nseg; q++) {
+    const int sg = BACK ? nseg - 1 - q : q, c = 128 * sg + 4 * lane, at = 128 * sg + 2 * lane;
+    const bool in = c < n, end = c + 4 == n;
+    Four bb = ld4(B + (in ? c : 0), 2);
+    const Four m4 = ld4(Xm + at, 64), p4 = ld4(Xp + at, 64), o4 = ld4(Xc + at, 64);
+    // the columns next to the segment (any column where there is none)
+    const int cl = sg > 0 ? pcol(128 * sg - 1) : 0, cr = sg + 1 < nseg ? 128 * (sg + 1) : 0;
+    const cx<float> el = sg > 0 ? ld1(Xm + cl) + ld1(Xp + cl) : wl, er = ld1(Xm + cr) + ld1(Xp + cr);
+    cx<float> w[4], y[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) w[t] = m4.v[t] + p4.v[t];
+    const cx<float> lft = pick(lane == 0, el, up_c(w[3], 1));
+    const cx<float> rgt = pick(end, wr, pick(lane == 31, er, dn_c(w[0], 1)));
+    const cx<float> s01 = w[0] + w[1], s12 = w[1] + w[2], s23 = w[2] + w[3];
+    y[0] = lft + s01;
+    y[1] = s01 + w[2];
+    y[2] = s12 + w[3];
+    y[3] = s23 + rgt;
+    // the old value of the next position (at the row's end the new first one,
+    // added below), the old value across the seam at the first
+    if (!BACK) {
+      const cx<float> nx = pick(lane == 31, ld1(Xc + cr), dn_c(o4.v[0], 1));
+      y[0] += o4.v[1];
+      y[1] += o4.v[2];
+      y[2] += o4.v[3];
+      if (!end) y[3] += nx;
+      if (c == 0) y[0] += old;
+    } else {
+      const cx<float> nx = pick(lane == 0, ld1(Xc + cl), up_c(o4.v[3], 1));
+      y[3] += o4.v[2];
+      y[2] += o4.v[1];
+      y[1] += o4.v[0];
+      if (c > 0) y[0] += nx;
+      if (end) y[3] += old;
+    }
+    if (phased) {
+#pragma unroll
+      for (int t = 0; t < 4; t++) bb.v[t] = bp * bb.v[t];
+    }
+#pragma unroll
+    for (int t = 0; t < 4; t++) y[t] = scal(0.375f, bb.v[t]) + scal(0.125f, y[t]);
+    if (!in) y[0] = y[1] = y[2] = y[3] = czero<float>();
+    // the first new value of the row and its way round to the last position
+    if (q == 0) first = BACK ? xfc * at_c(y[3], ((n - 4) & 127) / 4) : xf * at_c(y[0], 0);
+    if (BACK ? c == 0 : end) y[BACK ? 0 : 3] += scal(0.125f, first);
+    cx<float> s;
+    if (!BACK) {
+#pragma unroll
+      for (int t = 1; t < 4; t++) y[t] += scal(0.125f, y[t - 1]);
+      s = y[3];
+    } else {
+#pragma unroll
+      for (int t = 2; t >= 0; t--) y[t] += scal(0.125f, y[t + 1]);
+      s = y[0];
+    }
+    // scan of the runs: 16 positions back
+    float f = 1.0f / 4096.0f;
+#pragma unroll
+    for (int off = 1; off < 4; off *= 2) {
+      const cx<float> u = BACK ? dn_c(s, off) : up_c(s, off);
+      const float g = (BACK ? lane + off < 32 : lane >= off) ? f : 0.0f;
+      s += scal(g, u);
+      f *= f;
+    }
+    // the value before the lane's run: the neighbour lane's, and what the end
+    // of the segment before contributes
+    const int dl = BACK ? 31 - lane : lane;
+    const cx<float> prev = BACK ? dn_c(s, 1) : up_c(s, 1);
+    const cx<float> cin = scal(dl == 0 ? 0.0f : 1.0f, prev) + scal(pow84(dl), carry);
+    carry = at_c(s, BACK ? 0 : 31);
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      constexpr float w8[4] = {0.125f, 0.015625f, 0.001953125f, 0.000244140625f};
+      y[t] += scal(w8[BACK ? 3 - t : t], cin);
+    }
+    __syncwarp();
+    if (in) st4(Xc + at, 64, Four{{y[0], y[1], y[2], y[3]}});
+    __syncwarp();
+  }
+}
+
+template <bool POST>
+__global__ void __launch_bounds__(NBT, 2)
+    k_node_band(int n, int m, int K, int B, int nu, const double* __restrict__ ph, float third,
+                const float2* __restrict__ b, const float2* __restrict__ xin, const float2* __restrict__ xc,
+                float2* __restrict__ xout, float2* __restrict__ bc) {
+  extern __shared__ __align__(16) float2 sx[];
+  const int nb = (n + B - 1) / B, kv = blockIdx.x / nb, k = kv / m, nn = n * n, nc = n / 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = NBT / 32, nseg = (n + 127) / 128, NS = nseg * 128;
+  const int J0 = (int) (blockIdx.x - kv * nb) * B, J1 = J0 + B < n ? J0 + B : n;
+  // rows lo .. hi in shared memory (beyond 0 .. n-1 across the seam)
+  const int lo = J0 - 2 * nu - (POST ? 0 : 2), hi = J1 - 1 + 2 * nu + (POST ? 0 : 1);
+  const Seam<float> sm = seam_load<float>(ph, K, k, n);
+  const float2* bv = b + (size_t) kv * nn;
+  auto row_at = [&](int r) { return r < 0 ? r + n : r >= n ? r - n : r; };
+  auto X = [&](int r) { return sx + (r - lo) * NS; };
+  // ---- load (and prolongate into) the rows
+  for (int r = lo + warp; r <= hi; r += nw) {
+    const int j = row_at(r);
+    const bool out = j != r;
+    const cx<float> rp = r < 0 ? conjc(sm.yf) : sm.yf;
+    const float2* src = xin ? xin + (size_t) kv * nn + (size_t) j * n : nullptr;
+    const float2 *c0 = nullptr, *c1 = nullptr;
+    cx<float> p0 = mkc(1.0f, 0.0f), p1 = p0;
+    if (POST) {
+      // coarse rows J and J + 1 with the phases of rows outside the cell
+      const int J = r >= 0 ? r / 2 : -((1 - r) / 2), J2 = J + 1;
+      const float2* cv = xc + (size_t) kv * nc * nc;
+      c0 = cv + (size_t) (J < 0 ? J + nc : J >= nc ? J - nc : J) * nc;
+      c1 = cv + (size_t) (J2 < 0 ? J2 + nc : J2 >= nc ? J2 - nc : J2) * nc;
+      if (J < 0) p0 = conjc(sm.yf);
+      if (J >= nc) p0 = sm.yf;
+      if (J2 < 0) p1 = conjc(sm.yf);
+      if (J2 >= nc) p1 = sm.yf;
+    }
+    for (int c = 4 * lane, at = 2 * lane; c < n; c += 128, at += 128) {
+      Four t{{czero<float>(), czero<float>(), czero<float>(), czero<float>()}};
+      if (src) {
+        t = ld4(src + c, 2);
+        if (out)
+#pragma unroll
+          for (int q = 0; q < 4; q++) t.v[q] = rp * t.v[q];
+      }
+      if (POST) {
+        // coarse columns I, I + 1, I + 2
+        const int I = c / 2, I2 = I + 2 < nc ? I + 2 : 0;
+        const Two a0 = ld2(c0 + I);
+        cx<float> v0 = p0 * a0.a, v1 = p0 * a0.b, v2 = p0 * ld1(c0 + I2);
+        if (r & 1) {
+          const Two a1 = ld2(c1 + I);
+          v0 = scal(0.5f, v0 + p1 * a1.a);
+          v1 = scal(0.5f, v1 + p1 * a1.b);
+          v2 = scal(0.5f, v2 + p1 * ld1(c1 + I2));
+        }
+        if (I2 == 0) v2 = sm.xf * v2;
+        t.v[0] += v0;
+        t.v[1] += scal(0.5f, v0 + v1);
+        t.v[2] += v1;
+        t.v[3] += scal(0.5f, v1 + v2);
+      }
+      st4(X(r) + at, 64, t);
+    }
+  }
+  __syncthreads();
+  // ---- the sweeps
+  auto sweep_row = [&](int r) {
+    const int j = row_at(r);
+    band_row<POST>(n, X(r - 1), X(r), X(r + 1), bv + (size_t) j * n, j != r, r < 0 ? conjc(sm.yf) : sm.yf, sm.xf);
+  };
+#pragma unroll 1
+  for (int p = 1; p <= 2 * nu; p++) {
+    // forward: odd rows with row 0, then even rows with row n-1; backward the
+    // reverse.  A row next to a special one takes it along, in the sweep's order.
+    const bool odd = POST ? (p & 1) == 0 : (p & 1) == 1;
+    const bool before = POST ? !odd : odd;   // the special row comes before its neighbour
+    const int a = lo + p, e = hi - p, f0 = a + (((a & 1) != 0) != odd);
+#pragma unroll 1
+    for (int r = f0 + 2 * warp; r <= e; r += 2 * nw) {
+      const int j = row_at(r);
+      if (j == (odd ? n - 1 : 0)) continue;   // (the other phase's)
+      const bool next = j == (odd ? 1 : n - 2);
+      const int sp = odd ? r - 1 : r + 1;
+      const bool chain = next && sp >= a && sp <= e;
+      // up to two rows in turn, through one copy of the sweep's code
+#pragma unroll 1
+      for (int q = 0; q < 1 + (int) chain; q++) {
+        sweep_row(chain && (q == 0) == before ? sp : r);
+        __syncwarp();
+      }
+    }
+    // a special row that comes first, with its neighbour outside the range
+    if (before && warp == nw - 1)
+#pragma unroll 1
+      for (int q = 0; q < 2; q++) {
+        const int sp = odd ? q * n : q * n - 1, nbr = odd ? sp + 1 : sp - 1;
+        if (sp >= a && sp <= e && !(nbr >= a && nbr <= e)) sweep_row(sp);
+      }
+    __syncthreads();
+  }
+  // ---- results
+  float2* xo = xout + (size_t) kv * nn;
+  for (int r = J0 + warp; r < J1; r += nw)
+    for (int c = 4 * lane, at = 2 * lane; c < n; c += 128, at += 128) st4(xo + (size_t) r * n + c, 2, ld4(X(r) + at, 64));
+  if (!POST) {
+    // coarse rows J0/2 .. J1/2 - 1, the row in one or two parts.  t(c) =
+    // d(c, fj) + (d(c, fj-1) + d(c, fj+1)) / 2 with d = b - (9 x - the sum of
+    // nine) / 3; the coarse value is t(2I) + (t(2I-1) + t(2I+1)) / 2.  With h
+    // the sums of three columns, the x part of 3 t is row by row
+    // h/2, 3/2 (h - 3x), 2h - 9x, 3/2 (h - 3x), h/2: its partial sums stay small.
+    const int C0 = J0 / 2, parts = nseg > 1 ? 2 : 1, per = (nseg + parts - 1) / parts;
+    for (int tsk = warp; tsk < parts * (J1 - J0) / 2; tsk += nw) {
+      const int J = C0 + tsk / parts, sa = (tsk % parts) * per, sb = sa + per < nseg ? sa + per : nseg, fj = 2 * J;
+      constexpr float wh[5] = {0.5f, 1.5f, 2.0f, 1.5f, 0.5f}, wx[5] = {0.0f, 4.5f, 9.0f, 4.5f, 0.0f};
+      auto bphase = [&](int r) { return r < 0 ? conjc(sm.yf) : sm.yf; };
+      // t in the column before the part
+      cx<float> left = czero<float>();
+      {
+        const int c = sa > 0 ? 128 * sa - 1 : n - 1, pc = pcol(c), pm = pcol(c - 1), pp = c + 1 < n ? pcol(c + 1) : 0;
+        cx<float> acc = czero<float>();
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+          const int r = fj - 2 + q;
+          cx<float> g = ld1(X(r) + pp);
+          if (c + 1 == n) g = sm.xf * g;
+          const cx<float> x0 = ld1(X(r) + pc), h = ld1(X(r) + pm) + x0 + g;
+          acc += scal(wh[q], h) - scal(wx[q], x0);
+          if (q > 0 && q < 4) {
+            const int j = row_at(r);
+            cx<float> d = ld1(bv + (size_t) j * n + c);
+            if (j != r) d = bphase(r) * d;
+            left += scal(q == 2 ? 1.0f : 0.5f, d);
+          }
+        }
+        left += scal(third, acc);
+        if (sa == 0) left = conjc(sm.xf) * left;
+      }
+#pragma unroll 1
+      for (int sg = sa; sg < sb; sg++) {
+        const int c = 128 * sg + 4 * lane, at = 128 * sg + 2 * lane;
+        const int cl = sg > 0 ? pcol(128 * sg - 1) : pcol(n - 1), cr = sg + 1 < nseg ? 128 * (sg + 1) : 0;
+        const bool in = c < n, end = c + 4 == n;
+        Four acc{{czero<float>(), czero<float>(), czero<float>(), czero<float>()}}, t4 = acc;
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+          const int r = fj - 2 + q;
+          const float2* Xr = X(r);
+          const Four x4 = ld4(Xr + at, 64);
+          cx<float> el = ld1(Xr + cl), er = ld1(Xr + cr);
+          if (sg == 0) el = conjc(sm.xf) * el;
+          const cx<float> l = pick(lane == 0, el, up_c(x4.v[3], 1));
+          cx<float> g = pick(lane == 31, er, dn_c(x4.v[0], 1));
+          if (end) g = sm.xf * ld1(Xr);
+          const cx<float> s01 = x4.v[0] + x4.v[1], s23 = x4.v[2] + x4.v[3];
+          acc.v[0] += scal(wh[q], l + s01) - scal(wx[q], x4.v[0]);
+          acc.v[1] += scal(wh[q], s01 + x4.v[2]) - scal(wx[q], x4.v[1]);
+          acc.v[2] += scal(wh[q], x4.v[1] + s23) - scal(wx[q], x4.v[2]);
+          acc.v[3] += scal(wh[q], s23 + g) - scal(wx[q], x4.v[3]);
+          if (q > 0 && q < 4) {
+            const int j = row_at(r);
+            Four d = ld4(bv + (size_t) j * n + (in ? c : 0), 2);
+            if (j != r)
+#pragma unroll
+              for (int u = 0; u < 4; u++) d.v[u] = bphase(r) * d.v[u];
+#pragma unroll
+            for (int u = 0; u < 4; u++) t4.v[u] += scal(q == 2 ? 1.0f : 0.5f, d.v[u]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) acc.v[u] = t4.v[u] + scal(third, acc.v[u]);
+        const cx<float> l = pick(lane == 0, left, up_c(acc.v[3], 1));
+        left = at_c(acc.v[3], 31);
+        if (in)
+          st2(bc + (size_t) kv * nc * nc + (size_t) J * nc + c / 2,
+              Two{acc.v[0] + scal(0.5f, l + acc.v[1]), acc.v[2] + scal(0.5f, acc.v[1] + acc.v[3])});
+      }
+    }
+  }
+}
+
+// [k][e][v] <-> [k][v][e] in tiles of 64 elements x m vectors, both sides in
+// 16-byte accesses where m is even (nn is)
+__global__ void __launch_bounds__(256) k_planar(int nn, int m, int to, const float2* __restrict__ src,
+                                                float2* __restrict__ dst) {
+  __shared__ float2 t[32 * 65];   // [v][e], a vector's elements 65 apart
+  const int k = blockIdx.y, e0 = blockIdx.x * 64, ne = nn - e0 < 64 ? nn - e0 : 64, len = ne * m;
+  const size_t base = (size_t) k * nn * m;
+  const float2* si = src + base + (size_t) e0 * m;
+  float2* di = dst + base + (size_t) e0 * m;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (to) {
+    if (m % 2 == 0)
+      for (int q = 2 * threadIdx.x; q < len; q += 512) {
+        const int e = q / m, v = q - e * m;
+        const float4 f = *reinterpret_cast<const float4*>(si + q);
+        t[v * 65 + e] = make_float2(f.x, f.y);
+        t[(v + 1) * 65 + e] = make_float2(f.z, f.w);
+      }
+    else
+      for (int q = threadIdx.x; q < len; q += 256) t[(q % m) * 65 + q / m] = si[q];
+    __syncthreads();
+    for (int v = w; v < m; v += 8) {
+      const int e = 2 * lane;
+      if (e < ne) {
+        const float2 a = t[v * 65 + e], c = t[v * 65 + e + 1];
+        *reinterpret_cast<float4*>(dst + base + (size_t) v * nn + e0 + e) = make_float4(a.x, a.y, c.x, c.y);
+      }
+    }
+  } else {
+    for (int v = w; v < m; v += 8) {
+      const int e = 2 * lane;
+      if (e < ne) {
+        const float4 f = *reinterpret_cast<const float4*>(src + base + (size_t) v * nn + e0 + e);
+        t[v * 65 + e] = make_float2(f.x, f.y);
+        t[v * 65 + e + 1] = make_float2(f.z, f.w);
+      }
+    }
+    __syncthreads();
+    if (m % 2 == 0)
+      for (int q = 2 * threadIdx.x; q < len; q += 512) {
+        const int e = q / m, v = q - e * m;
+        const float2 a = t[v * 65 + e], c = t[(v + 1) * 65 + e];
+        *reinterpret_cast<float4*>(di + q) = make_float4(a.x, a.y, c.x, c.y);
+      }
+    else
+      for (int q = threadIdx.x; q < len; q += 256) di[q] = t[(q % m) * 65 + q / m];
+  }
+}
+
+// rows per band: as many as two CTAs per SM hold, fewer (down to 8) where the
+// batch leaves SMs without a CTA; even, the last band not below 8 rows
+int band_rows(int n, int vecs, int halo) {
+  int B = (110 * 1024) / ((n + 127) / 128 * 128 * 8) - halo;
+  const int want = (int) (((size_t) n * vecs + 607) / 608);   // four CTAs per SM
+  if (B > want) B = want;
+  if (B > n / 2) B = n / 2;
+  B &= ~1;
+  if (B < 8) B = 8;
+  for (int q = B; q >= 8; q -= 2)
+    if (n % q == 0 || n % q >= 8) return q;
+  while (n % B != 0 && n % B < 8) B += 2;
+  return B;
 }
 
 size_t cycle_smem(int n0, int top, int prec) {
@@ -302,11 +707,11 @@ size_t cycle_smem(int n0, int top, int prec) {
 }
 
 template <typename S, typename R, typename MS>
-int run(int n0, int top, int m, int K, int nu, int cycles, int zero, const double* ph, const void* ainv, int prec,
+int run(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar, const double* ph, const void* ainv, int prec,
         const void* b, void* x, cudaStream_t st) {
   const size_t smem = cycle_smem(n0, top, prec);
   cudaFuncSetAttribute(k_node_vcycle<S, R, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-  k_node_vcycle<S, R, MS><<<(unsigned) K * m, NCT, smem, st>>>(n0, top, m, K, nu, cycles, zero, ph, make_sc(1.0 / 3.0),
+  k_node_vcycle<S, R, MS><<<(unsigned) K * m, NCT, smem, st>>>(n0, top, m, K, nu, cycles, zero, planar, ph, make_sc(1.0 / 3.0),
                                                                (const MS*) ainv, (const S*) b, (S*) x);
   MX_CHECK_LAUNCH();
   return 0;
@@ -325,13 +730,49 @@ extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
   return l;
 }
 
-extern "C" int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, const double* ph,
-                               const double* ainv, const void* ainv_c64, int prec, const void* b, void* x, mx_stream s) {
+extern "C" int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
+                               const double* ph, const double* ainv, const void* ainv_c64, int prec, const void* b, void* x, mx_stream s) {
   cudaStream_t st = (cudaStream_t) s;
   if (prec == MX_C64) {
-    if (ainv_c64) return run<float2, float, float2>(n0, top, m, K, nu, cycles, zero, ph, ainv_c64, prec, b, x, st);
-    return run<float2, float, double2>(n0, top, m, K, nu, cycles, zero, ph, ainv, prec, b, x, st);
+    if (ainv_c64) return run<float2, float, float2>(n0, top, m, K, nu, cycles, zero, planar, ph, ainv_c64, prec, b, x, st);
+    return run<float2, float, double2>(n0, top, m, K, nu, cycles, zero, planar, ph, ainv, prec, b, x, st);
   }
-  if (prec == MX_C128) return run<double2, double, double2>(n0, top, m, K, nu, cycles, zero, ph, ainv, prec, b, x, st);
-  return run<cdd, dd, double2>(n0, top, m, K, nu, cycles, zero, ph, ainv, prec, b, x, st);
+  if (prec == MX_C128) return run<double2, double, double2>(n0, top, m, K, nu, cycles, zero, planar, ph, ainv, prec, b, x, st);
+  return run<cdd, dd, double2>(n0, top, m, K, nu, cycles, zero, planar, ph, ainv, prec, b, x, st);
+}
+
+// c64 levels of 100 to 512 nodes a side (a row of more columns would leave the
+// bands mostly halo), at most two sweeps each way
+extern "C" int mxk_node_band_ok(int n, int m, int nu, int prec) {
+  return prec == MX_C64 && n > 96 && n <= 512 && n % 4 == 0 && nu >= 1 && nu <= 2 && m <= 32;
+}
+
+extern "C" int mxk_node_band_pre(int n, int m, int K, int nu, const double* ph, const void* b, const void* xin, void* xout,
+                                 void* bc, mx_stream s) {
+  const int halo = 4 * nu + 3, B = band_rows(n, K * m, halo), nb = (n + B - 1) / B;
+  const size_t smem = (size_t) (B + halo) * ((n + 127) / 128 * 128) * sizeof(float2);
+  cudaFuncSetAttribute(k_node_band<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  k_node_band<false><<<(unsigned) nb * K * m, NBT, smem, (cudaStream_t) s>>>(
+      n, m, K, B, nu, ph, (float) (1.0 / 3.0), (const float2*) b, (const float2*) xin, nullptr, (float2*) xout, (float2*) bc);
+  MX_CHECK_LAUNCH();
+  return 0;
+}
+
+extern "C" int mxk_node_band_post(int n, int m, int K, int nu, const double* ph, const void* b, const void* xin,
+                                  const void* xc, void* xout, mx_stream s) {
+  const int halo = 4 * nu, B = band_rows(n, K * m, halo), nb = (n + B - 1) / B;
+  const size_t smem = (size_t) (B + halo) * ((n + 127) / 128 * 128) * sizeof(float2);
+  cudaFuncSetAttribute(k_node_band<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  k_node_band<true><<<(unsigned) nb * K * m, NBT, smem, (cudaStream_t) s>>>(
+      n, m, K, B, nu, ph, (float) (1.0 / 3.0), (const float2*) b, (const float2*) xin, (const float2*) xc, (float2*) xout,
+      nullptr);
+  MX_CHECK_LAUNCH();
+  return 0;
+}
+
+extern "C" int mxk_node_planar(int n, int m, int K, int to, const void* src, void* dst, mx_stream s) {
+  const int nn = n * n;
+  k_planar<<<dim3((nn + 63) / 64, K), 256, 0, (cudaStream_t) s>>>(nn, m, to, (const float2*) src, (float2*) dst);
+  MX_CHECK_LAUNCH();
+  return 0;
 }

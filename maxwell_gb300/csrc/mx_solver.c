@@ -116,6 +116,7 @@ struct mxg_solver {
   int order;                          /* earlier waves a warm start combines (1, 2 or 3) */
   int all_columns;                    /* Ritz basis with every search column (refinement) */
   int device;                         /* the CUDA device the solver lives on */
+  int planar[MAXL];                   /* the lifting of level l runs on planar node vectors */
 };
 
 #define L_(x) do { int e_ = (x); s->launches++; if (e_) return e_; } while (0)
@@ -131,6 +132,8 @@ static mxk_kappa kap(const mxg_solver *s, int l)
 
 static size_t elen(const mxg_solver *s, int l) { return (size_t) s->K * 2 * s->n[l] * s->n[l] * s->m; }
 static size_t nlen(const mxg_solver *s, int l) { return (size_t) s->K * s->n[l] * s->n[l] * s->m; }
+
+static int planar_level(const mxg_solver *s, int l);
 
 static int dalloc(void **p, size_t bytes)
 {
@@ -281,6 +284,7 @@ mxg_solver *mxg_solver_new(const mxg_solve_opts *o, const double *kappa_fine)
     goto fail;
   s->E0 = s->E;
   s->P0 = s->P;
+  for(l = 1; l <= o->L; l++) s->planar[l] = planar_level(s, l);
   s->gscratch_bytes = (size_t) K * 256 * (ns * (ns + 1) / 2) * 4 * sizeof(double);
   if(s->gscratch_bytes > ((size_t) 1 << 30)) s->gscratch_bytes = (size_t) 1 << 30;
   if(dalloc((void **) &s->gscratch, s->gscratch_bytes)) goto fail;
@@ -460,25 +464,56 @@ static int vcycle_e(mxg_solver *s, int top)
   return 0;
 }
 
-/* The level from which the node V-cycle runs in one launch (0: none; with
- * profiling on, the finest level keeps its launches, which carry the events). */
-static int fused_node_level(const mxg_solver *s, int top)
+/* `cycles` node V-cycles of the levels up to l in one launch */
+static int fused_node_cycles(mxg_solver *s, int l, int cycles, int zero, int planar)
 {
-  int c = mxk_node_vcycle_top(s->n0, top, s->pg);
-  return s->prof && c == s->L ? 0 : c;
+  int on = prof_begin(s, l, MXG_KT_NODE_GS, (double) nlen(s, l) * (zero ? 2.0 : 3.0) * mxk_elem_size(s->pg));
+  L_(mxk_node_vcycle(s->n0, l, s->m, s->K, s->o.smoother_steps, cycles, zero, planar, s->ph, s->an_inv, s->an_inv_f,
+                     s->pg, s->bg[l], s->xg[l], s->st));
+  prof_end(s, on);
+  return 0;
 }
 
-static int fused_node_cycles(mxg_solver *s, int l, int cycles, int zero)
+/* The lifting of level l runs on planar vectors when every level of its node
+ * V-cycle has a kernel of that form: the bands of the fine levels, one launch
+ * for the rest (the opt-in tiled sweep keeps its own layout).  Decided when
+ * the solver is made: its CUDA graphs hold the choice. */
+static int planar_level(const mxg_solver *s, int l)
 {
-  L_(mxk_node_vcycle(s->n0, l, s->m, s->K, s->o.smoother_steps, cycles, zero, s->ph, s->an_inv, s->an_inv_f, s->pg,
-                     s->bg[l], s->xg[l], s->st));
+  int lc, q;
+  if(s->pg != MX_C64 || mxk_node_gs_oop_ok(s->n[l], s->m, s->pg)) return 0;
+  lc = mxk_node_vcycle_top(s->n0, l, s->pg);
+  if(lc == 0) return 0;
+  for(q = lc + 1; q <= l; q++)
+    if(!mxk_node_band_ok(s->n[q], s->m, s->o.smoother_steps, s->pg)) return 0;
+  return 1;
+}
+
+/* vcycle_node2d on planar vectors, x[top] from zero where zero is set: one
+ * launch per fine level on the way down (sweeps, residual, restriction) and
+ * up (prolongation, sweeps), one for the levels below */
+static int vcycle_n_planar(mxg_solver *s, int top, int zero)
+{
+  int l, on, lc = mxk_node_vcycle_top(s->n0, top, s->pg), nu = s->o.smoother_steps;
+  for(l = top; l > lc; l--) {
+    const void *xin = l == top && !zero ? s->xg[l] : 0;
+    on = prof_begin(s, l, MXG_KT_NODE_GS, (double) nlen(s, l) * (xin ? 3.25 : 2.25) * mxk_elem_size(s->pg));
+    L_(mxk_node_band_pre(s->n[l], s->m, s->K, nu, s->ph, s->bg[l], xin, s->dg[l], s->bg[l - 1], s->st));
+    prof_end(s, on);
+  }
+  TRY(fused_node_cycles(s, lc, 1, lc < top || zero, 1));
+  for(l = lc + 1; l <= top; l++) {
+    on = prof_begin(s, l, MXG_KT_NODE_GS, (double) nlen(s, l) * 3.25 * mxk_elem_size(s->pg));
+    L_(mxk_node_band_post(s->n[l], s->m, s->K, nu, s->ph, s->bg[l], s->dg[l], s->xg[l - 1], s->xg[l], s->st));
+    prof_end(s, on);
+  }
   return 0;
 }
 
 /* vcycle_node2d (node2d.c:1352-1389) on bg[top], xg[top] */
 static int vcycle_n(mxg_solver *s, int top)
 {
-  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg, lc = fused_node_level(s, top);
+  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg, lc = mxk_node_vcycle_top(s->n0, top, pg);
   for(l = top; l > lc; l--) {
     int n = s->n[l];
     TRY(node_smooth(s, l, 0, nu));
@@ -487,7 +522,7 @@ static int vcycle_n(mxg_solver *s, int top)
     if(l - 1 > lc || lc == 0) L_(mxk_zero(pg, s->xg[l - 1], nlen(s, l - 1), s->st));
   }
   if(lc > 0)
-    TRY(fused_node_cycles(s, lc, 1, lc < top));
+    TRY(fused_node_cycles(s, lc, 1, lc < top, 0));
   else
     L_(mxk_coarse_apply(s->n0 * s->n0, m, K, s->an_inv, s->an_inv_f, pg, s->bg[0], s->xg[0], s->st));
   for(l = lc + 1; l <= top; l++) {
@@ -538,7 +573,13 @@ static int run_graphed(mxg_solver *s, int l, cudaGraphExec_t *exec, long *nlaunc
 static int lift_body(mxg_solver *s, int l)
 {
   int i;
-  if(l > 0 && fused_node_level(s, l) == l) return fused_node_cycles(s, l, s->o.gradient_steps, 1);
+  if(l > 0 && mxk_node_vcycle_top(s->n0, l, s->pg) == l)
+    return fused_node_cycles(s, l, s->o.gradient_steps, 1, s->planar[l]);
+  if(s->planar[l]) {
+    for(i = 0; i < s->o.gradient_steps; i++)
+      TRY(vcycle_n_planar(s, l, i == 0));
+    return 0;
+  }
   L_(mxk_zero(s->pg, s->xg[l], nlen(s, l), s->st));
   for(i = 0; i < s->o.gradient_steps; i++)
     TRY(vcycle_n(s, l));
@@ -549,9 +590,9 @@ static int lift(mxg_solver *s, int l, int py, void *y)
 {
   int n = s->n[l];
   if(s->o.gradient_steps <= 0) return 0;
-  L_(mxk_adjgradient(n, s->m, s->K, s->ph, 1.0, 1, 0.0, py, y, s->pg, s->bg[l], s->st));
+  L_(mxk_adjgradient(n, s->m, s->K, s->ph, 1.0, 1, 0.0, s->planar[l], py, y, s->pg, s->bg[l], s->st));
   TRY(run_graphed(s, l, &s->glift[l], &s->glift_n[l], lift_body));
-  L_(mxk_gradient(n, s->m, s->K, s->ph, -1.0, s->pg, s->xg[l], py, y, s->st));
+  L_(mxk_gradient(n, s->m, s->K, s->ph, -1.0, s->planar[l], s->pg, s->xg[l], py, y, s->st));
   return 0;
 }
 
@@ -566,10 +607,10 @@ static int hcycle_e(mxg_solver *s, int top)
     for(i = 0; i < nu; i++)
       L_(mxk_edge_gs_point(n, m, K, s->ph, kap(s, l), 1.0, 1.0, 0, pg, s->b[l], s->x[l], s->st));
     L_(mxk_edge_apply(n, m, K, s->ph, kap(s, l), -1.0, -1.0, 0, 1.0, pg, s->x[l], pg, s->b[l], s->d[l], s->st));
-    L_(mxk_adjgradient(n, m, K, s->ph, 1.0, 0, 0.0, pg, s->d[l], pg, s->bg[l], s->st));
+    L_(mxk_adjgradient(n, m, K, s->ph, 1.0, 0, 0.0, 0, pg, s->d[l], pg, s->bg[l], s->st));
     L_(mxk_zero(pg, s->xg[l], nlen(s, l), s->st));
     TRY(node_smooth(s, l, 0, nu));
-    L_(mxk_gradient(n, m, K, s->ph, 1.0, pg, s->xg[l], pg, s->x[l], s->st));
+    L_(mxk_gradient(n, m, K, s->ph, 1.0, 0, pg, s->xg[l], pg, s->x[l], s->st));
     L_(mxk_edge_apply(n, m, K, s->ph, kap(s, l), -1.0, -1.0, 0, 1.0, pg, s->x[l], pg, s->b[l], s->d[l], s->st));
     L_(mxk_zero(pg, s->b[l - 1], elen(s, l - 1), s->st));
     L_(mxk_edge_restrict(n / 2, m, K, s->ph, 1.0, pg, s->d[l], s->b[l - 1], s->st));
@@ -580,10 +621,10 @@ static int hcycle_e(mxg_solver *s, int top)
     int n = s->n[l];
     L_(mxk_edge_prolong(n / 2, m, K, s->ph, 1.0, pg, s->x[l - 1], s->x[l], s->st));
     L_(mxk_edge_apply(n, m, K, s->ph, kap(s, l), -1.0, -1.0, 0, 1.0, pg, s->x[l], pg, s->b[l], s->d[l], s->st));
-    L_(mxk_adjgradient(n, m, K, s->ph, 1.0, 0, 0.0, pg, s->d[l], pg, s->bg[l], s->st));
+    L_(mxk_adjgradient(n, m, K, s->ph, 1.0, 0, 0.0, 0, pg, s->d[l], pg, s->bg[l], s->st));
     L_(mxk_zero(pg, s->xg[l], nlen(s, l), s->st));
     TRY(node_smooth(s, l, 1, nu));
-    L_(mxk_gradient(n, m, K, s->ph, 1.0, pg, s->xg[l], pg, s->x[l], s->st));
+    L_(mxk_gradient(n, m, K, s->ph, 1.0, 0, pg, s->xg[l], pg, s->x[l], s->st));
     for(i = 0; i < nu; i++)
       L_(mxk_edge_gs_point(n, m, K, s->ph, kap(s, l), 1.0, 1.0, 1, pg, s->b[l], s->x[l], s->st));
   }

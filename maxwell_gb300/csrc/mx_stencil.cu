@@ -1392,13 +1392,54 @@ __global__ void k_gradient(int n, int m, int K, const double* __restrict__ ph, S
   Store<SE, R>::st(py, Store<SE, R>::ld(py) + scal(a, gy));
 }
 
-template <typename SE, typename SV, typename R>
+// the same from a planar c64 vector ([k][v][j][i]): a CTA stages the nodes of
+// its stretch of a row (GP_STEPS times the block's sites) and of the row
+// above for all vectors
+constexpr int GP_STEPS = 4;
+template <typename SE, typename R>
+__global__ void k_gradient_planar(int n, int m, int K, const double* __restrict__ ph, Sc alpha,
+                                  const float2* __restrict__ vin, SE* __restrict__ e) {
+  // block (m, rows): x = vector, y = site; grid (stretches x rows of nodes, K)
+  extern __shared__ float2 sg[];   // [2][m][W]
+  const int k = blockIdx.y, rows = blockDim.y, len = rows * GP_STEPS, W = len + 1, str = (n + len - 1) / len;
+  const int j = blockIdx.x / str, i0 = (blockIdx.x - j * str) * len, tid = threadIdx.y * m + threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = (rows * m + 31) >> 5, last = rows * m - 1 - 32 * warp;
+  const int lanes = last < 31 ? last + 1 : 32;   // (the last warp may be short)
+  const Seam<R> sm = seam_load<R>(ph, K, k, n);
+  for (int q = warp; q < 2 * m; q += nw) {
+    const int u = q >= m, v = u ? q - m : q;
+    const float2* src = vin + ((size_t) k * m + v) * n * n + (size_t) (j + u == n ? 0 : j + u) * n;
+    for (int d = lane; d < W && i0 + d <= n; d += lanes) sg[q * W + d] = src[i0 + d == n ? 0 : i0 + d];
+  }
+  __syncthreads();
+  Lay L{n, m, K};
+  const R a = sget<R>(alpha);
+  const int v = threadIdx.x;
+#pragma unroll
+  for (int t = 0; t < GP_STEPS; t++) {
+    const int d = t * rows + threadIdx.y, i = i0 + d;
+    if (i >= n) break;
+    const float2* s0 = sg + v * W + d;
+    const cx<R> c = Store<float2, R>::ld(s0);
+    cx<R> r = Store<float2, R>::ld(s0 + 1), u = Store<float2, R>::ld(s0 + m * W);
+    if (i == n - 1) r = sm.xf * r;
+    if (j == n - 1) u = sm.yf * u;
+    SE* px = e + L.edge(k, 0, j, i, v);
+    SE* py = e + L.edge(k, 1, j, i, v);
+    Store<SE, R>::st(px, Store<SE, R>::ld(px) + scal(a, r - c));
+    Store<SE, R>::st(py, Store<SE, R>::ld(py) + scal(a, u - c));
+  }
+}
+
+// PLANAR: the result goes to a planar c64 vector, turned in shared memory
+template <typename SE, typename SV, typename R, bool PLANAR>
 __global__ void k_adjgradient(int n, int m, int K, const double* __restrict__ ph, Sc alpha, int mass,
                               Sc sixth, Sc cv, int has_cv, const SE* __restrict__ e, SV* __restrict__ vout) {
   // block (m, rows): x = vector, y = site; grid.y = k-point
   int k = blockIdx.y, v = threadIdx.x;
   int site = blockIdx.x * blockDim.y + threadIdx.y;
-  if (site >= n * n) return;
+  if (!PLANAR && site >= n * n) return;
+  if (PLANAR && site >= n * n) site = n * n - 1;   // (not written)
   int i = site % n, j = site / n;
   Lay L{n, m, K};
   const SE* eb = e + L.edge(k, 0, 0, 0, v);
@@ -1432,8 +1473,17 @@ __global__ void k_adjgradient(int n, int m, int K, const double* __restrict__ ph
     EAcc<SE, R> E{eb, n, m, seam_load<R>(ph, K, k, n)};
     s = E(0, i - 1, j) - E(0, i, j) + E(1, i, j - 1) - E(1, i, j);
   }
-  SV* p = vout + L.node(k, j, i, v);
   cx<R> o = scal(sget<R>(alpha), s);
+  if constexpr (PLANAR) {
+    __shared__ float2 turn[256 + 32];
+    const int rows = blockDim.y, tid = threadIdx.y * m + v, s0 = blockIdx.x * rows;
+    Store<float2, R>::st(turn + v * (rows + 1) + threadIdx.y, o);
+    __syncthreads();
+    const int tv = tid / rows, ts = tid - tv * rows;
+    if (s0 + ts < n * n) vout[((size_t) k * m + tv) * n * n + s0 + ts] = turn[tv * (rows + 1) + ts];
+    return;
+  }
+  SV* p = vout + L.node(k, j, i, v);
   if (has_cv) o += scal(sget<R>(cv), Store<SV, R>::ld(p));
   Store<SV, R>::st(p, o);
 }
@@ -1963,11 +2013,24 @@ extern "C" int mxk_node_restrict(int nc, int m, int K, const double* ph, double 
   return MX_BY_PREC(prec, L_node_restrict, nc, m, K, ph, alpha, f, c, (cudaStream_t) s);
 }
 
-extern "C" int mxk_gradient(int n, int m, int K, const double* ph, double alpha, int pv, const void* v,
+extern "C" int mxk_gradient(int n, int m, int K, const double* ph, double alpha, int planar, int pv, const void* v,
                             int pe, void* e, mx_stream s) {
   dim3 g = grd2((size_t) n * n, m, K), b = blk2(m);
   cudaStream_t st = (cudaStream_t) s;
   Sc a = make_sc(alpha);
+  if (planar) {
+    if (pv != MX_C64) return (int) cudaErrorInvalidValue;
+    const int len = (int) b.y * GP_STEPS;
+    const dim3 gp((unsigned) (n * ((n + len - 1) / len)), K);
+    const size_t sm = sizeof(float2) * 2 * m * (len + 1);
+#define MX_GP(SE, R) k_gradient_planar<SE, R><<<gp, b, sm, st>>>(n, m, K, ph, a, (const float2*) v, (SE*) e)
+    if (pe == MX_C64) MX_GP(float2, float);
+    else if (pe == MX_CDD) MX_GP(cdd, dd);
+    else MX_GP(double2, double);
+#undef MX_GP
+    MX_CHECK_LAUNCH();
+    return 0;
+  }
 #define MX_G(SV, SE, R) k_gradient<SV, SE, R><<<g, b, 0, st>>>(n, m, K, ph, a, (const SV*) v, (SE*) e)
   if (pv == MX_C64 && pe == MX_C64) MX_G(float2, float2, float);
   else if (pv == MX_C128 && pe == MX_C128) MX_G(double2, double2, double);
@@ -1980,21 +2043,27 @@ extern "C" int mxk_gradient(int n, int m, int K, const double* ph, double alpha,
   return 0;
 }
 
-extern "C" int mxk_adjgradient(int n, int m, int K, const double* ph, double alpha, int mass, double cv,
+extern "C" int mxk_adjgradient(int n, int m, int K, const double* ph, double alpha, int mass, double cv, int planar,
                                int pe, const void* e, int pv, void* v, mx_stream s) {
   dim3 g = grd2((size_t) n * n, m, K), b = blk2(m);
   cudaStream_t st = (cudaStream_t) s;
   Sc a = make_sc(alpha), sixth = make_sc(1.0 / 6.0), c = make_sc(cv);
   int has = cv != 0.0;
-#define MX_AG(SE, SV, R) \
-  k_adjgradient<SE, SV, R><<<g, b, 0, st>>>(n, m, K, ph, a, mass, sixth, c, has, (const SE*) e, (SV*) v)
-  if (pe == MX_C64 && pv == MX_C64) MX_AG(float2, float2, float);
-  else if (pe == MX_C128 && pv == MX_C128) MX_AG(double2, double2, double);
+  if (planar && (pv != MX_C64 || has)) return (int) cudaErrorInvalidValue;
+#define MX_AG(SE, SV, R, PL) \
+  k_adjgradient<SE, SV, R, PL><<<g, b, 0, st>>>(n, m, K, ph, a, mass, sixth, c, has, (const SE*) e, (SV*) v)
   // G^H M e of a nearly divergence-free eigenvector is a sum with heavy
   // cancellation: it is formed in float-float and only then rounded to c64
-  else if (pe == MX_CDD && pv == MX_C64) MX_AG(cdd, float2, dd);
-  else if (pe == MX_CDD && pv == MX_CDD) MX_AG(cdd, cdd, dd);
-  else if (pe == MX_C128 && pv == MX_C64) MX_AG(double2, float2, double);
+  if (planar) {
+    if (pe == MX_C64) MX_AG(float2, float2, float, true);
+    else if (pe == MX_CDD) MX_AG(cdd, float2, dd, true);
+    else MX_AG(double2, float2, double, true);
+  }
+  else if (pe == MX_C64 && pv == MX_C64) MX_AG(float2, float2, float, false);
+  else if (pe == MX_C128 && pv == MX_C128) MX_AG(double2, double2, double, false);
+  else if (pe == MX_CDD && pv == MX_C64) MX_AG(cdd, float2, dd, false);
+  else if (pe == MX_CDD && pv == MX_CDD) MX_AG(cdd, cdd, dd, false);
+  else if (pe == MX_C128 && pv == MX_C64) MX_AG(double2, float2, double, false);
   else return (int) cudaErrorInvalidValue;
 #undef MX_AG
   MX_CHECK_LAUNCH();

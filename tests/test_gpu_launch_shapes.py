@@ -164,3 +164,48 @@ def test_gram_and_combination_block_sizes(n, m, K, prec):
     got = y.get()
     for k in range(K):
         assert rel(got[k], coef[k].T @ u[k]) < {mx.C128: 1e-14, mx.CDD: 1e-13, mx.C64: 2e-6}[prec] * m
+
+
+@pytest.mark.parametrize("n0, L, m, K, nu", [(8, 4, 2, 2, 2), (10, 4, 3, 1, 1), (8, 5, 1, 2, 2), (6, 5, 2, 1, 2),
+                                             (8, 6, 1, 1, 2), (14, 3, 5, 1, 2)])
+def test_node_vcycle_bands(oracle, n0, L, m, K, nu):
+    """c64 node V-cycles whose fine levels run in bands of rows (112 to 512
+    nodes a side; one and two sweeps each way, bands of 8 rows and more, the
+    bands at the seam in both directions, a last segment of a row that is not
+    full) against the cycle put together from the oracle's sweeps."""
+    rng = np.random.default_rng(n0 + L)
+    n = n0 << L
+    fac = FACTORS[[0, 2]][:K]
+    grids = [mx.Grid(n, K, None, fac)]
+    for _ in range(L):
+        grids.append(grids[-1].coarsen())
+    grids = grids[::-1]
+    import ctypes as C
+    b, x, d = ([mx.Node(g, m, mx.C64) for g in grids] for _ in range(3))
+    b[L].put(cv(rng, K, m, n * n))
+    x[L].put(cv(rng, K, m, n * n))
+    rhs, start = b[L].get(), x[L].get()
+    A, info = mx.Matrix(n0 * n0, K), np.zeros(K, np.int32)
+    mx.check(mx.lib().densematrix_node2d_gpu(1, grids[0].h, A.h))
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    arr = [(C.c_void_p * (L + 1))(*[o.h for o in objs]) for objs in (b, x, d)]
+    mx.check(mx.lib().vcycle_node2d_gpu(L, nu, A.h, *arr))
+    got = x[L].get()
+    assert np.array_equal(b[L].get(), rhs)
+
+    def cycle(l, f, bl, xl):
+        nl = n0 << l
+        if l == 0:
+            return np.linalg.solve(oracle.dense_node(n0, *f, 1), bl)
+        for _ in range(nu):
+            xl = oracle.gs_node(nl, *f, 1.0, 0, bl, xl)
+        r = oracle.addeval_node(nl, *f, -1.0, xl, bl)
+        c = oracle.restrict_node(nl // 2, *f, 1.0, r, np.zeros(nl * nl // 4, complex))
+        xl = oracle.prolong_node(nl // 2, *f, 1.0, cycle(l - 1, f, c, np.zeros_like(c)), xl)
+        for _ in range(nu):
+            xl = oracle.gs_node(nl, *f, 1.0, 1, bl, xl)
+        return xl
+
+    for k in range(K):
+        for v in {0, m - 1}:
+            assert rel(got[k, v], cycle(L, fac[k], rhs[k, v], start[k, v])) < 1e-4
