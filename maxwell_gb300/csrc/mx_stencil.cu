@@ -16,6 +16,7 @@
 #include "mx_internal.h"
 #include "maxwell_gb300.h"
 
+#include <algorithm>
 #include <atomic>
 
 using namespace mx;
@@ -710,7 +711,7 @@ __global__ void k_edge_gs_point(int n, int m, int K, const double* __restrict__ 
 // vector, k-point), the same local solve as the row sweep.  A forward sweep
 // takes the colours (0,0), (1,0), (0,1), (1,1), a backward sweep the reverse
 // order; the two colours of one vertex-row parity share a launch
-// (k_edge_gs_rowpair).  The iterates differ from the reference's row order; both are
+// (k_edge_gs_rowpair for c64, k_edge_gs_rowseg for FP64 and float-float).  The iterates differ from the reference's row order; both are
 // convergent splittings of the same operator, so the eigenpairs the solver
 // converges to are the same.
 // ------------------------------------------------------------------
@@ -825,6 +826,159 @@ __global__ void k_edge_gs_rowpair(int n, int m, int K, const double* __restrict_
   }
   if (threadIdx.y == 0)
     afw_patch<S, R>(n, m, K, ph, kap, ftab, axy_s, mm_s, s8_s, is8_s, (F + n - 1) % n, j, k, v, b, x);
+}
+
+// 2 alpha n^2 kappa of a patch's four cells and the factors of its 4x4 matrix
+template <typename R> struct alignas(16) AfwSlot {
+  R wLL, wUL, wLR, wUR;
+  R l20, l21, i0, i1, i2, pad[3];
+};
+constexpr int AFW_TAB_BYTES = 48 * 1024;   // most shared memory that a CTA's table of patches takes
+constexpr int AFW_PARTS = 4;               // CTAs that share a row
+
+// afw_patch with the weights and factors from a table
+template <typename S, typename R>
+__device__ __forceinline__ void afw_patch_tab(int n, int m, int K, const double* __restrict__ ph,
+                                          const AfwSlot<R>& slot, const Sc& mm_s, const Sc& is8_s, int i, int j, int k, int v, const S* __restrict__ b,
+                                          S* x) {
+  const AfwSlot<R> f = slot;
+  const R mm = sget<R>(mm_s), is8 = sget<R>(is8_s), four = rc<R>(4.0f), quarter = rc<R>(0.25f);
+  const bool inner = i > 0 && i < n - 1 && j > 0 && j < n - 1;
+  cx<R> xa0, xa1, xa2, xb0, xb1, xb2, ya0, ya1, yb0, yb1, yc0, yc1, bx0, bx1, by0, by1;
+  Seam<R> seam;
+  // x(i, j) of the vector; a row, a plane and a column on
+  const ptrdiff_t row = (ptrdiff_t) n * m, plane = row * n;
+  const size_t o = Lay{n, m, K}.edge(k, 0, j, i, v);
+  S* xp = x + o;
+  if (inner) {
+    auto at = [](const S* p) { return Store<S, R>::ld(p); };
+    const S *bp = b + o, *xl = xp - m;
+    bx0 = at(bp - m); bx1 = at(bp); by0 = at(bp + plane - row); by1 = at(bp + plane);
+    xa0 = at(xl - row); xa1 = at(xl); xa2 = at(xl + row);
+    xb0 = at(xp - row); xb1 = at(xp); xb2 = at(xp + row);
+    ya0 = at(xl + plane - row); ya1 = at(xl + plane);
+    yb0 = at(xp + plane - row); yb1 = at(xp + plane);
+    yc0 = at(xp + plane - row + m); yc1 = at(xp + plane + m);
+  } else {
+    Lay L{n, m, K};
+    seam = seam_load<R>(ph, K, k, n);
+    EAcc<S, R> X{x + L.edge(k, 0, 0, 0, v), n, m, seam}, B{b + L.edge(k, 0, 0, 0, v), n, m, seam};
+    xa0 = X(0, i - 1, j - 1); xa1 = X(0, i - 1, j); xa2 = X(0, i - 1, j + 1);
+    xb0 = X(0, i, j - 1); xb1 = X(0, i, j); xb2 = X(0, i, j + 1);
+    ya0 = X(1, i - 1, j - 1); ya1 = X(1, i - 1, j);
+    yb0 = X(1, i, j - 1); yb1 = X(1, i, j);
+    yc0 = X(1, i + 1, j - 1); yc1 = X(1, i + 1, j);
+    bx0 = B(0, i - 1, j); bx1 = B(0, i, j); by0 = B(1, i, j - 1); by1 = B(1, i, j);
+  }
+  const cx<R> cLL = scal(f.wLL, xa0 - xa1 - ya0 + yb0);
+  const cx<R> cUL = scal(f.wUL, xa1 - xa2 - ya1 + yb1);
+  const cx<R> cLR = scal(f.wLR, xb0 - xb1 - yb0 + yc0);
+  const cx<R> cUR = scal(f.wUR, xb1 - xb2 - yb1 + yc1);
+  // b less the mass term; the curls join in the four combinations, where they cancel from the last, the
+  // gradient of the vertex, without the rounding of terms of size n^2
+  const cx<R> g0 = bx0 - scal(mm, scal(four, xa1) + (xa2 + xa0));
+  const cx<R> g1 = bx1 - scal(mm, scal(four, xb1) + (xb2 + xb0));
+  const cx<R> g2 = by0 - scal(mm, scal(four, yb0) + (yc0 + ya0));
+  const cx<R> g3 = by1 - scal(mm, scal(four, yb1) + (yc1 + ya1));
+  const cx<R> sx = g0 + g1, dx = g0 - g1, sy = g2 + g3, dy = g2 - g3;
+  cx<R> c0 = sx + sy - (cUL - cLR), c1 = sx - sy + (cLL - cUR), c2 = dx - dy + (cLL - cUL + cUR - cLR), c3 = dx + dy;
+  c2 -= scal(f.l20, c0) + scal(f.l21, c1);
+  c0 = scal(f.i0, c0);
+  c1 = scal(f.i1, c1);
+  c2 = scal(f.i2, c2);
+  c3 = scal(is8, c3);
+  c1 -= scal(f.l21, c2);
+  c0 -= scal(f.l20, c2);
+  const cx<R> s01 = c0 + c1, d01 = c0 - c1, s23 = c2 + c3, d23 = c2 - c3;
+  xa1 += scal(quarter, s01 + s23);
+  xb1 += scal(quarter, s01 - s23);
+  yb0 += scal(quarter, d01 - d23);
+  yb1 += scal(quarter, d01 + d23);
+  if (inner) {
+    Store<S, R>::st(xp - m, xa1);
+    Store<S, R>::st(xp, xb1);
+    Store<S, R>::st(xp + plane - row, yb0);
+    Store<S, R>::st(xp + plane, yb1);
+  } else {
+    S* xb = x + Lay{n, m, K}.edge(k, 0, 0, 0, v);
+    st_edge<S, R>(xb, n, m, seam, 0, i - 1, j, xa1);
+    st_edge<S, R>(xb, n, m, seam, 0, i, j, xb1);
+    st_edge<S, R>(xb, n, m, seam, 1, i, j - 1, yb0);
+    st_edge<S, R>(xb, n, m, seam, 1, i, j, yb1);
+  }
+}
+
+// k_edge_gs_rowpair for FP64 and float-float: the same patches in the same
+// order, a vertex row per cluster of nseg CTAs that take an equal part
+// [p0, p1) of it each.  The second-colour patch of p0 needs the last
+// first-colour patch of the part before it and comes last, after a barrier
+// of the cluster; no barrier parts a chunk's second colour from the next
+// chunk's first, they do not interact.
+//
+// The FP64 unit bounds it (2 FMA per clock and SM; an instruction of a warp
+// holds its quarter's for 64 cycles).  So the weights and factors of the
+// patches, with five divisions each, are made once per patch and not once
+// per vector: a table in shared memory of T chunks at a time; and the rows
+// are cut, since 128 CTAs of one row each (n = 64, four k-points) left 24 SMs
+// idle and walked their chunks one after another.  Sweep of 12 FP64 vectors
+// at four k-points: 64^2 281 -> 120 us, 128^2 755 -> 342; of 8 at two, 512^2
+// 2486 -> 1393; float-float 256^2 x 16 at four 1460 -> 1019.  With the row
+// uncut 210, 560 and 1827 us, cut in two 146, 421 and 1481.  64 registers
+// (some spilled) and four CTAs an SM beat 128 and two (64^2 119 against 128
+// us, 256^2 x 8 at four 758 against 871).  c64 waits for memory and not for
+// arithmetic: there the table's fill and the cut cost more than they save
+// (512^2, 16 k-points x 16: 1239 us without, 1287 to 1490 with).
+template <typename S, typename R>
+__global__ void __launch_bounds__(256, 4)
+k_edge_gs_rowseg(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap, Sc axy_s, Sc mm_s,
+                 Sc s8_s, Sc is8_s, int cj, int rev, int nseg, int T, const S* __restrict__ b, S* x) {
+  // block (m, P): x = vector, y = patch lane; grid (rows of the parity x nseg, K)
+  extern __shared__ __align__(16) unsigned char afw_tab_raw[];
+  AfwSlot<R>* tab = reinterpret_cast<AfwSlot<R>*>(afw_tab_raw);
+  const int k = blockIdx.y, v = threadIdx.x, ty = threadIdx.y, P = blockDim.y, h = n / 2, SL = 2 * P * T + 1;
+  const int rowi = blockIdx.x / nseg, sg = blockIdx.x - rowi * nseg;
+  const int j = 2 * rowi + cj, F = rev;
+  const int p0 = (int) ((long long) h * sg / nseg), p1 = (int) ((long long) h * (sg + 1) / nseg);
+  const bool single = p1 - p0 <= P;
+  // slot s < 2PT: column 2c + F - 1 + s; slot 2PT: the second-colour patch of p0
+  auto fill = [&](int c) {
+    for (int s = ty * m + v; s < SL; s += m * P) {
+      if (s < SL - 1 && c + s / 2 >= p1) continue;
+      const int i = wrapi(s < SL - 1 ? 2 * c + F - 1 + s : 2 * p0 + F - 1, n);
+      const R axy = sget<R>(axy_s);
+      const R kLL = kap(i - 1, j - 1), kUL = kap(i - 1, j), kLR = kap(i, j - 1), kUR = kap(i, j);
+      AfwSlot<R> e;
+      const R two = rc<R>(2.0f) * axy;
+      e.wLL = two * kLL; e.wUL = two * kUL; e.wLR = two * kLR; e.wUR = two * kUR;
+      afw_factors<R>(kLL, kUL, kLR, kUR, axy, sget<R>(s8_s), e.l20, e.l21, e.i0, e.i1, e.i2);
+      tab[s] = e;
+    }
+  };
+  for (int c = p0, u = 0; c < p1; c += P, u++) {
+    if (u == T) u = 0;
+    if (u == 0) {
+      if (c > p0) __syncthreads();
+      fill(c);
+      __syncthreads();
+    }
+    const bool last = c + P >= p1;
+    const AfwSlot<R>* t = tab + 2 * P * u;
+    if (c + ty < p1)
+      afw_patch_tab<S, R>(n, m, K, ph, t[2 * ty + 1], mm_s, is8_s, 2 * (c + ty) + F, j, k, v, b, x);
+    if (last && nseg > 1) {
+      asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+    const int r = last ? p1 - c : P;
+    for (int l = ty; l < r + (last && !single); l += P) {
+      const int q = l < r ? c + l : p0;
+      if (q == p0 && l < r && !single) continue;
+      const int i = 2 * q + F - 1;
+      afw_patch_tab<S, R>(n, m, K, ph, l < r ? t[2 * l] : tab[SL - 1], mm_s, is8_s, i < 0 ? i + n : i, j, k, v, b,
+                          x);
+    }
+  }
 }
 
 // ------------------------------------------------------------------
@@ -1936,13 +2090,33 @@ extern "C" int mxk_edge_gs(int n, int m, int K, const double* ph, mxk_kappa kap,
 template <typename S, typename R>
 static int L_edge_gs_rowpair(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha, double beta,
                              int cj, int rev, const void* b, void* x, cudaStream_t st) {
-  const float4* ftab = (sizeof(R) == 4 && kap.afw && kap.afw_alpha == alpha && kap.afw_beta == beta)
-                           ? (const float4*) kap.afw : nullptr;
-  k_edge_gs_rowpair<S, R><<<dim3(n / 2, K), blk2(m), 0, st>>>(
-      n, m, K, ph, make_kap<R>(kap, n), ftab, make_sc(alpha * (double) n * (double) n), make_sc(beta / 6.0),
-      make_sc(8.0 * beta / 6.0), make_sc(6.0 / (8.0 * beta)), cj, rev, (const S*) b, (S*) x);
-  MX_CHECK_LAUNCH();
-  return 0;
+  if constexpr (sizeof(S) > 8) {
+    const int h = n / 2, nseg = h >= AFW_PARTS ? AFW_PARTS : 1, part = (h + nseg - 1) / nseg;
+    const int pairs = (AFW_TAB_BYTES / (int) sizeof(AfwSlot<R>) - 1) / 2;   // first-colour patches of a table
+    const int P = std::min({256 / m, part, pairs}), T = std::min(pairs / P, (part + P - 1) / P);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = nseg;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(h * nseg, K);
+    cfg.blockDim = dim3(m, P);
+    cfg.dynamicSmemBytes = (2 * P * T + 1) * sizeof(AfwSlot<R>);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return (int) cudaLaunchKernelEx(&cfg, k_edge_gs_rowseg<S, R>, n, m, K, ph, make_kap<R>(kap, n),
+                                    make_sc(alpha * (double) n * (double) n), make_sc(beta / 6.0),
+                                    make_sc(8.0 * beta / 6.0), make_sc(6.0 / (8.0 * beta)), cj, rev, nseg, T,
+                                    (const S*) b, (S*) x);
+  } else {
+    const float4* ftab = kap.afw && kap.afw_alpha == alpha && kap.afw_beta == beta ? (const float4*) kap.afw : nullptr;
+    k_edge_gs_rowpair<S, R><<<dim3(n / 2, K), blk2(m), 0, st>>>(
+        n, m, K, ph, make_kap<R>(kap, n), ftab, make_sc(alpha * (double) n * (double) n), make_sc(beta / 6.0),
+        make_sc(8.0 * beta / 6.0), make_sc(6.0 / (8.0 * beta)), cj, rev, (const S*) b, (S*) x);
+    MX_CHECK_LAUNCH();
+    return 0;
+  }
 }
 
 extern "C" int mxk_edge_gs_colour(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,

@@ -58,6 +58,44 @@ def test_row_smoother_chunks(oracle, n, m, K, prec, direction):
             assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 1e-11)
 
 
+@pytest.mark.parametrize("n, m, K", [(2, 3, 1), (6, 16, 2), (8, 1, 1), (10, 24, 1), (74, 7, 2), (130, 32, 1),
+                                     (64, 12, 3)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_colour_smoother_parts(oracle, n, m, K, prec, direction):
+    """The patch smoother in four colours, rows cut in four: rows too short
+    to cut (2, 6), parts of one patch (8), parts that differ by one (10, 74,
+    130), parts of one chunk and of several (130 with 8 patch lanes)."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    g = mx.Grid(n, K, kap, FACTORS[:K])
+    b, x = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    eb, ex = mx.Edge(g, m, prec, b), mx.Edge(g, m, prec, x)
+    mx.check(mx.lib().gscolour_edge2d_gpu(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h, direction))
+    got = ex.get()
+    for k in range(K):
+        for v in {0, m // 2, m - 1}:
+            want = oracle.gs_edge_colour(n, kap, *FACTORS[k], 1.0, 0.8, direction, b[k, v], x[k, v])
+            assert rel(got[k, v], want) < 1e-11
+
+
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD])
+def test_colour_smoother_table_refill(prec):
+    """Parts of more patches than their table holds (257 against 255): one
+    vector alone and the same vector among four, whose chunks and tables are
+    cut at other patches, agree to the bit."""
+    rng = np.random.default_rng(29)
+    n = 2052
+    g = mx.Grid(n, 1, 1.0 / (1.0 + 11.0 * rng.random(n * n)), FACTORS[:1])
+    b, x = cv(rng, 1, 1, 2 * n * n), cv(rng, 1, 1, 2 * n * n)
+    got = []
+    for m in (1, 4):
+        eb, ex = [mx.Edge(g, m, prec, np.repeat(a, m, axis=1)) for a in (b, x)]
+        mx.check(mx.lib().gscolour_edge2d_gpu(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h, 0))
+        got.append(ex.get()[0, m - 1])
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("n0, L, m", [(4, 2, 6), (6, 2, 9), (10, 1, 12), (12, 1, 8)])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_coarse_grid_sizes(oracle, n0, L, m, precision):
