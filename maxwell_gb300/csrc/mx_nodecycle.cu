@@ -19,10 +19,16 @@
 // n-2 of the even ones, so one warp takes each such pair in sequence and a
 // sweep is two phases with a barrier each.
 //
-// Bound by the latency of a phase (shared loads, scan, barrier; FP64 blocks by
-// the FP64 rate of the K m SMs it occupies).  One cycle of the levels 64 .. 8,
+// Bound by the latency of a phase (shared loads, scan, barrier), FP64 blocks by
+// the FP64 rate of the K m SMs it would occupy: few FP64 vectors take a
+// cluster of CTAs each, which share the rows and nodes of a phase; every CTA
+// keeps a copy of the levels and writes its part to all of them.  One cycle of the levels 64 .. 8,
 // 8 k-points x 16 c64 vectors: 66 us against about 460 us in 62 launches; five
-// cycles from 64 of 4 x 12 FP64 vectors 2.2 ms against 9.9 ms.
+// cycles from 64 of 4 x 12 FP64 vectors 1.6 ms against 9.9 ms.
+#include <cooperative_groups.h>
+
+#include <type_traits>
+
 #include "mx_common.cuh"
 #include "mx_internal.h"
 
@@ -43,10 +49,27 @@ __device__ __forceinline__ double from0(double v) { return __shfl_sync(0xfffffff
 __device__ __forceinline__ dd from0(dd v) { return dd_make(from0(v.hi), from0(v.lo)); }
 template <typename R> __device__ __forceinline__ cx<R> up_c(cx<R> v, int d) { return mkc(up_r(v.re, d), up_r(v.im, d)); }
 
+// The CTAs of a cluster that share a vector: each holds every level, does a
+// part of the rows and nodes and writes its results to all copies
+template <bool CLU> struct Team {
+  unsigned size, rank;
+  __device__ __forceinline__ void sync() const {
+    if constexpr (CLU) asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+    else __syncthreads();
+  }
+  template <typename T> __device__ __forceinline__ void put(T* p, const T& v) const {
+    if constexpr (CLU) {
+      for (unsigned q = 0; q < size; q++) *cooperative_groups::this_cluster().map_shared_rank(p, q) = v;
+    } else {
+      *p = v;
+    }
+  }
+};
+
 // one row of one sweep by a warp; EDGE: row 0 or n-1, whose neighbour rows
 // cross the seam
-template <typename R, int LR, bool EDGE>
-__device__ void gs_row(int n, int j, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm) {
+template <typename R, int LR, bool EDGE, typename TM>
+__device__ void gs_row(int n, int j, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm, const TM& team) {
   const int lane = threadIdx.x & 31, t0 = lane * LR;
   const R eighth = rc<R>(0.125f), c38 = rc<R>(0.375f);
   const cx<R>* Xm = X + (j == 0 ? n - 1 : j - 1) * n;
@@ -107,14 +130,14 @@ __device__ void gs_row(int n, int j, int back, cx<R>* X, const cx<R>* B, const S
 #pragma unroll
   for (int q = 0; q < LR; q++) {
     carry = scal(eighth, carry);
-    if (t0 + q < n) Xc[at(t0 + q)] = y[q] + carry;
+    if (t0 + q < n) team.put(Xc + at(t0 + q), y[q] + carry);
   }
 }
 
 // one sweep by the CTA; ends at a barrier
-template <typename R, int LR>
-__device__ void sweep(int n, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm) {
-  const int warp = threadIdx.x >> 5, nw = NCT / 32;
+template <typename R, int LR, typename TM>
+__device__ void sweep(int n, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm, const TM& team) {
+  const int warp = (threadIdx.x >> 5) * team.size + team.rank, nw = NCT / 32 * team.size;
 #pragma unroll 1
   for (int ph = 0; ph < 2; ph++) {
     // forward: row 0 and the odd rows, then the even rows and row n-1;
@@ -123,38 +146,38 @@ __device__ void sweep(int n, int back, cx<R>* X, const cx<R>* B, const Seam<R>& 
     if (warp == 0) {
       const int edge = odd ? 0 : n - 1, next = odd ? 1 : n - 2;
       if (ph == 0) {
-        gs_row<R, LR, true>(n, edge, back, X, B, sm);
+        gs_row<R, LR, true>(n, edge, back, X, B, sm, team);
         __syncwarp();
-        gs_row<R, LR, false>(n, next, back, X, B, sm);
+        gs_row<R, LR, false>(n, next, back, X, B, sm, team);
       } else {
-        gs_row<R, LR, false>(n, next, back, X, B, sm);
+        gs_row<R, LR, false>(n, next, back, X, B, sm, team);
         __syncwarp();
-        gs_row<R, LR, true>(n, edge, back, X, B, sm);
+        gs_row<R, LR, true>(n, edge, back, X, B, sm, team);
       }
     } else {
       // the group's other rows: 3, 5 .. n-3 or 2, 4 .. n-4
-      for (int r = warp - 1; r < n / 2 - 2; r += nw - 1) gs_row<R, LR, false>(n, (odd ? 3 : 2) + 2 * r, back, X, B, sm);
+      for (int r = warp - 1; r < n / 2 - 2; r += nw - 1) gs_row<R, LR, false>(n, (odd ? 3 : 2) + 2 * r, back, X, B, sm, team);
     }
-    __syncthreads();
+    team.sync();
   }
 }
 
-template <typename R>
-__device__ void smooth(int n, int nu, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm) {
+template <typename R, typename TM>
+__device__ void smooth(int n, int nu, int back, cx<R>* X, const cx<R>* B, const Seam<R>& sm, const TM& team) {
   for (int q = 0; q < nu; q++) {
-    if (n <= 32) sweep<R, 1>(n, back, X, B, sm);
-    else if (n <= 64) sweep<R, 2>(n, back, X, B, sm);
-    else sweep<R, 3>(n, back, X, B, sm);
+    if (n <= 32) sweep<R, 1>(n, back, X, B, sm, team);
+    else if (n <= 64) sweep<R, 2>(n, back, X, B, sm, team);
+    else sweep<R, 3>(n, back, X, B, sm, team);
   }
 }
 
 // bc = restriction of b - L x, xc = 0
-template <typename R>
+template <typename R, typename TM>
 __device__ void restrict_residual(int n, const cx<R>* X, const cx<R>* B, cx<R>* Xc, cx<R>* Bc, const Seam<R>& sm,
-                                  const Sc& third_s) {
+                                  const Sc& third_s, const TM& team) {
   const int nc = n / 2;
   const R third = sget<R>(third_s), half = rc<R>(0.5f), nine = rc<R>(9.0f);
-  for (int e = threadIdx.x; e < nc * nc; e += NCT) {
+  for (int e = threadIdx.x + team.rank * NCT; e < nc * nc; e += NCT * team.size) {
     const int I = e % nc, J = e / nc, fi = 2 * I, fj = 2 * J;
     cx<R> out;
     auto body = [&](const auto& V, const auto& W) {
@@ -197,18 +220,18 @@ __device__ void restrict_residual(int n, const cx<R>* X, const cx<R>* B, cx<R>* 
       };
       body(wrapped(X), wrapped(B));
     }
-    Bc[e] = out;
-    Xc[e] = czero<R>();
+    team.put(Bc + e, out);
+    team.put(Xc + e, czero<R>());
   }
-  __syncthreads();
+  team.sync();
 }
 
 // x += P xc, bilinear
-template <typename R>
-__device__ void prolong(int n, cx<R>* X, const cx<R>* Xc, const Seam<R>& sm) {
+template <typename R, typename TM>
+__device__ void prolong(int n, cx<R>* X, const cx<R>* Xc, const Seam<R>& sm, const TM& team) {
   const int nc = n / 2;
   const R half = rc<R>(0.5f);
-  for (int e = threadIdx.x; e < nc * nc; e += NCT) {
+  for (int e = threadIdx.x + team.rank * NCT; e < nc * nc; e += NCT * team.size) {
     const int I = e % nc, J = e / nc;
     const bool wi = I == nc - 1, wj = J == nc - 1;
     const int I1 = wi ? 0 : I + 1, J1 = wj ? 0 : J + 1;
@@ -218,12 +241,12 @@ __device__ void prolong(int n, cx<R>* X, const cx<R>* Xc, const Seam<R>& sm) {
     cx<R>* p0 = X + 2 * J * n + 2 * I;
     cx<R>* p1 = p0 + n;
     const cx<R> h0 = scal(half, c00 + c10), h1 = scal(half, c01 + c11);
-    p0[0] += c00;
-    p0[1] += h0;
-    p1[0] += scal(half, c00 + c01);
-    p1[1] += scal(half, h0 + h1);
+    team.put(p0, p0[0] + c00);
+    team.put(p0 + 1, p0[1] + h0);
+    team.put(p1, p1[0] + scal(half, c00 + c01));
+    team.put(p1 + 1, p1[1] + scal(half, h0 + h1));
   }
-  __syncthreads();
+  team.sync();
 }
 
 // x = Ainv b on the coarsest level: N rows, the columns split over NCT / N
@@ -245,12 +268,14 @@ __device__ void coarse_solve(int N, const MS* __restrict__ ainv, cx<R>* X, const
   __syncthreads();
 }
 
-template <typename S, typename R, typename MS>
+template <typename S, typename R, typename MS, bool CLU>
 __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero,
                                                    int planar, const double* __restrict__ ph, Sc third,
                                                    const MS* __restrict__ ainv, const S* __restrict__ b, S* x) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  const int v = blockIdx.x % m, k = blockIdx.x / m, n = n0 << top, nn = n * n;
+  const unsigned cl = CLU ? gridDim.x / (unsigned) (K * m) : 1u;
+  const Team<CLU> team{cl, CLU ? blockIdx.x % cl : 0u};
+  const int kv = blockIdx.x / team.size, v = kv % m, k = kv / m, n = n0 << top, nn = n * n;
   // level l: x, then b; the top level first
   cx<R>* part = reinterpret_cast<cx<R>*>(sm_raw);
   cx<R>* X = part + NCT;
@@ -268,7 +293,7 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
     X[nn + e] = Store<S, R>::ld(bk + e * es);
     X[e] = zero ? czero<R>() : Store<S, R>::ld(xk + e * es);
   }
-  __syncthreads();
+  team.sync();
   for (int c = 0; c < cycles; c++) {
 #pragma unroll 1
     for (int l = top; l > 0; l--) {
@@ -276,8 +301,8 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
       cx<R>*Xl = level(l), *Xc = level(l - 1);
       Seam<R> sm = sm0;
       sm.n = nl;
-      smooth<R>(nl, nu, 0, Xl, Xl + nl * nl, sm);
-      restrict_residual<R>(nl, Xl, Xl + nl * nl, Xc, Xc + nl * nl / 4, sm, third);
+      smooth<R>(nl, nu, 0, Xl, Xl + nl * nl, sm, team);
+      restrict_residual<R>(nl, Xl, Xl + nl * nl, Xc, Xc + nl * nl / 4, sm, third, team);
     }
     {
       cx<R>* X0 = level(0);
@@ -289,11 +314,11 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
       cx<R>* Xl = level(l);
       Seam<R> sm = sm0;
       sm.n = nl;
-      prolong<R>(nl, Xl, level(l - 1), sm);
-      smooth<R>(nl, nu, 1, Xl, Xl + nl * nl, sm);
+      prolong<R>(nl, Xl, level(l - 1), sm, team);
+      smooth<R>(nl, nu, 1, Xl, Xl + nl * nl, sm, team);
     }
   }
-  for (int e = threadIdx.x; e < nn; e += NCT) Store<S, R>::st(xk + e * es, X[e]);
+  for (int e = threadIdx.x + team.rank * NCT; e < nn; e += NCT * team.size) Store<S, R>::st(xk + e * es, X[e]);
 }
 
 // ------------------------------------------------------------------
@@ -710,11 +735,31 @@ template <typename S, typename R, typename MS>
 int run(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar, const double* ph, const void* ainv, int prec,
         const void* b, void* x, cudaStream_t st) {
   const size_t smem = cycle_smem(n0, top, prec);
-  cudaFuncSetAttribute(k_node_vcycle<S, R, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-  k_node_vcycle<S, R, MS><<<(unsigned) K * m, NCT, smem, st>>>(n0, top, m, K, nu, cycles, zero, planar, ph, make_sc(1.0 / 3.0),
-                                                               (const MS*) ainv, (const S*) b, (S*) x);
-  MX_CHECK_LAUNCH();
-  return 0;
+  // FP64 vectors over a cluster of CTAs where SMs are left for it: cycle of
+  // levels 64 .. 8 of 48 vectors 510 us on one CTA each, 380 on two; of 16,
+  // 509, 379 and on four 348; of one, 502, 374 and 342.  Three CTAs for 48 no
+  // longer run side by side (693 us).  Levels 32 .. 8: 197 and 180; 16, 8: 87
+  // and 89.  c64 and float-float do not wait for the arithmetic unit: 63 -> 95
+  // and 331 -> 371 us on two.
+  int cl = 1;
+  if (prec == MX_C128 && n0 << top >= 32) cl = K * m <= 16 ? 4 : K * m <= 64 ? 2 : 1;
+  auto kern = k_node_vcycle<S, R, MS, false>;
+  if constexpr (std::is_same<R, double>::value)
+    if (cl > 1) kern = k_node_vcycle<S, R, MS, true>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cl;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned) K * m * cl);
+  cfg.blockDim = dim3(NCT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = cl > 1;
+  return (int) cudaLaunchKernelEx(&cfg, kern, n0, top, m, K, nu, cycles, zero, planar, ph, make_sc(1.0 / 3.0),
+                                  (const MS*) ainv, (const S*) b, (S*) x);
 }
 
 }  // namespace

@@ -114,17 +114,19 @@ def test_coarse_grid_sizes(oracle, n0, L, m, precision):
     assert np.abs(lam[:, :ie] - lam_o[:, :ie]).max() / lam_o[:, :ie].max() < 1e-8
 
 
-@pytest.mark.parametrize("n0, L, m, K", [(4, 1, 1, 1), (8, 3, 3, 2), (10, 2, 2, 1), (6, 4, 1, 2), (8, 4, 2, 1)])
+@pytest.mark.parametrize("n0, L, m, K", [(4, 1, 1, 1), (8, 3, 3, 2), (10, 2, 2, 1), (6, 4, 1, 2), (8, 4, 2, 1),
+                                         (8, 3, 20, 1), (8, 2, 32, 3)])
 @pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
 def test_node_vcycle_levels(oracle, n0, L, m, K, prec):
     """Node V-cycles from a given start on grids that run in one launch down
     to the coarse solve (8, 64, 40 and 96 nodes a side: one, two and three
     positions per lane, rows shorter than the warp; in FP64 96 and 128 keep
-    upper levels of their own) against the cycle put together from the
-    oracle's sweeps, residual and transfers."""
+    upper levels of their own; four, two or one CTA for each FP64 vector)
+    against the cycle put together from the oracle's sweeps, residual and
+    transfers."""
     rng = np.random.default_rng(n0 + L)
     n = n0 << L
-    fac = FACTORS[[0, 2]][:K]
+    fac = FACTORS[[0, 2, 0]][:K]
     grids = [mx.Grid(n, K, None, fac)]
     for _ in range(L):
         grids.append(grids[-1].coarsen())
