@@ -785,8 +785,12 @@ extern "C" int mxk_block_residual(int n, int m, int K, const double* ph, mxk_kap
   if (m > 32) return (int) cudaErrorInvalidValue;
   size_t nsite = (size_t) n * n;
   // about residual_sites sites per thread, so that the per-thread double
-  // reduction at the end stays small against the sweep
-  const size_t per = (size_t) rows * g_tuning.residual_sites;
+  // reduction at the end stays small against the sweep; fewer where that
+  // would leave less than four CTAs an SM (32^2 x 12 at 8 k-points: 2 x 8 CTAs
+  // of 32 sites a thread 100 us, 49 x 8 of one 22; 64^2 FP64 x 12 at
+  // four: 203 us, 65)
+  const size_t most = nsite * K / ((size_t) rows * 4 * sm_count()) + 1;
+  const size_t per = (size_t) rows * (most < (size_t) g_tuning.residual_sites ? most : (size_t) g_tuning.residual_sites);
   unsigned G = (unsigned) ((nsite + per - 1) / per);
   if (G < 1) G = 1;
   if (G > 4096) G = 4096;
