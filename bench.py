@@ -227,12 +227,12 @@ def fp64_residual_check(mx, n, kap, fac, lam, vec) -> float:
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per timed
-# sequence at 32 k-points, scaled by 8 from ncu captures at 4 k-points (the
-# full 32-k workload holds > 30 GB on the device): node GS sweep
-# (profiles/node_gs_512x512_k4_ncu.md), AFW sweep
-# (profiles/afw_rowpair_512x512_k4_ncu.md), Gram
+# sequence at 32 k-points, scaled from ncu captures at 8 or 4 k-points (the
+# full 32-k workload holds > 30 GB on the device): node smoothing launch
+# (profiles/node_band_512x512_k8_ncu.md, two sweeps and the restriction), AFW
+# sweep (profiles/afw_rowpair_512x512_k4_ncu.md), Gram
 # (profiles/block_gram_split_512x512_k4_ncu.md)
-TRAFFIC_32K = {"node_gs": 8 * 484.0e6, "afw": 8 * 2 * 648.1e6, "gram": 8 * 3.501e9}
+TRAFFIC_32K = {"node_gs": 4 * 843.6e6, "afw": 8 * 2 * 648.1e6, "gram": 8 * 3.501e9}
 
 
 def run_ours(args):
@@ -286,8 +286,8 @@ def run_ours(args):
     res_fp64 = fp64_residual_check(mx, n, kap, fac, lam, vec)
     del vec
 
-    # roofline kernels: one more solve with the finest level's node GS
-    # sweeps, AFW sweeps and Gram launches bracketed by CUDA events on the
+    # roofline kernels: one more solve with the finest level's node smoothing
+    # launches, AFW sweeps and Gram launches bracketed by CUDA events on the
     # solver's stream (the timed solves replay CUDA graphs, whose inner
     # launches carry no events)
     s.profile(True)
@@ -354,8 +354,9 @@ def run_ours(args):
                 "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": int(launches),
         "clocks": clock,
-        "roofline": roof("node_gs", "k_node_gs_warp + k_node_gs_rowpar (node Gauss-Seidel of the gradient "
-                                    "lifting, finest level)", "one node GS sweep (4 launches)",
+        "roofline": roof("node_gs", "k_node_band (node Gauss-Seidel of the gradient lifting with the "
+                                    "residual's restriction or the prolongation, finest level)",
+                         "one side of a node V-cycle's finest level (two sweeps and the transfer, one launch)",
                          TRAFFIC_32K["node_gs"]),
         "roofline_more": [roof("gram", "k_block_gram_split + k_gram_reduce (Gram matrices of [E X P])",
                                "one Gram of the Ritz step", TRAFFIC_32K["gram"]),
