@@ -88,6 +88,62 @@ __global__ void k_hpd_inverse(int N, double* a, int* info) {
   if (threadIdx.x == 0 && info) info[blockIdx.x] = bad;
 }
 
+// The same for matrices whose lower triangle fits into shared memory, by the
+// symmetric sweep operator: with d = a_pp, a_ij -= a_ip a_pj / d, a_ip /= d,
+// a_pp = -1 / d keep the matrix Hermitian, and sweeping every p leaves -A^-1.
+// Half the arithmetic of the Gauss-Jordan step, which the FP64 unit of one SM
+// bounds, no index division per entry and no round trip to L2.  A warp takes
+// whole columns (packed, column j from its diagonal on).  Orders 128 and 64
+// (n0 = 8), together: 5.2 -> 3.1 ms.
+constexpr int SWT = 512;
+__host__ __device__ inline size_t sweep_smem(int N) { return ((size_t) N * (N + 1) / 2 + 2 * (size_t) N) * sizeof(Z); }
+
+__global__ void __launch_bounds__(SWT) k_hpd_inverse_sweep(int N, double* a, int* info) {
+  extern __shared__ double sm[];
+  Z* f = reinterpret_cast<Z*>(sm);
+  Z* g = f + N;
+  Z* L = g + N;
+  double* A = a + (size_t) blockIdx.x * 2 * N * N;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = SWT / 32;
+  auto col = [&](int j) { return L + j * N - j * (j + 1) / 2; };   // col(j)[i] = a_ij, i >= j
+  for (int j = warp; j < N; j += nw)
+    for (int i = j + lane; i < N; i += 32) col(j)[i] = AT(A, N, i, j);
+  __syncthreads();
+  int bad = 0;
+  for (int p = 0; p < N; p++) {
+    const double d = col(p)[p].re;
+    if (!(d > 0.0)) bad = p + 1;
+    if ((int) threadIdx.x < N) {
+      const int i = threadIdx.x;
+      const double inv = 1.0 / d;
+      const Z v = i >= p ? col(p)[i] : zconj(col(i)[p]);
+      f[i] = v;
+      g[i] = i == p ? zmk(-inv, 0.0) : zmk(v.re * inv, v.im * inv);
+    }
+    __syncthreads();
+    for (int j = warp; j < N; j += nw) {
+      Z* c = col(j);
+      if (j == p) {
+        for (int i = j + lane; i < N; i += 32) c[i] = g[i];
+      } else {
+        const Z gj = g[j];
+        for (int i = j + lane; i < N; i += 32) {
+          const Z v = zsub(c[i], zcmul(gj, f[i]));
+          c[i] = i == p ? zconj(gj) : v;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = warp; j < N; j += nw)
+    for (int i = j + lane; i < N; i += 32) {
+      const Z v = col(j)[i];
+      AT(A, N, i, j) = zmk(-v.re, i == j ? 0.0 : -v.im);
+      if (i > j) AT(A, N, j, i) = zmk(-v.re, v.im);
+    }
+  if (threadIdx.x == 0 && info) info[blockIdx.x] = bad;
+}
+
 // ------------------------------------------------------------------
 // y_k = Ainv_k x_k on a level-0 block: the block of one k-point is a
 // row-major N x m matrix (dense row r at offset r*m)
@@ -574,7 +630,13 @@ size_t jacobi_smem(int N) {
 }  // namespace
 
 extern "C" int mxk_hpd_inverse(int N, int K, double* a, int* info, mx_stream s) {
-  k_hpd_inverse<<<K, DT, 2 * N * sizeof(Z), (cudaStream_t) s>>>(N, a, info);
+  const size_t smem = sweep_smem(N);
+  if (smem <= 208 * 1024) {   // orders up to 160
+    cudaFuncSetAttribute(k_hpd_inverse_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    k_hpd_inverse_sweep<<<K, SWT, smem, (cudaStream_t) s>>>(N, a, info);
+  } else {
+    k_hpd_inverse<<<K, DT, 2 * N * sizeof(Z), (cudaStream_t) s>>>(N, a, info);
+  }
   MX_CHECK_LAUNCH();
   return 0;
 }

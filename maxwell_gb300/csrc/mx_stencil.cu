@@ -711,9 +711,10 @@ __global__ void k_edge_gs_point(int n, int m, int K, const double* __restrict__ 
 // vector, k-point), the same local solve as the row sweep.  A forward sweep
 // takes the colours (0,0), (1,0), (0,1), (1,1), a backward sweep the reverse
 // order; the two colours of one vertex-row parity share a launch
-// (k_edge_gs_rowpair for c64, k_edge_gs_rowseg for FP64 and float-float).  The iterates differ from the reference's row order; both are
-// convergent splittings of the same operator, so the eigenpairs the solver
-// converges to are the same.
+// (k_edge_gs_rowpair for c64, k_edge_gs_rowseg for FP64 and float-float).  The
+// iterates differ from the reference's row order; both are convergent
+// splittings of the same operator, so the eigenpairs the solver converges to
+// are the same.
 // ------------------------------------------------------------------
 template <typename S, typename R>
 __device__ __forceinline__ void st_edge(S* base, int n, int m, const Seam<R>& seam, int p, int i, int j, cx<R> v) {

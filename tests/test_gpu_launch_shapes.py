@@ -249,3 +249,25 @@ def test_node_vcycle_bands(oracle, n0, L, m, K, nu):
     for k in range(K):
         for v in {0, m - 1}:
             assert rel(got[k, v], cycle(L, fac[k], rhs[k, v], start[k, v])) < 1e-4
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 64, 97, 160, 161])
+def test_hermitian_inverse_orders(n):
+    """The explicit inverse behind potrf_matrix_gpu: orders below, at and
+    above a warp, the largest whose triangle is held in shared memory and the
+    first beyond it; and the report of pivots that are not positive.
+    Condition numbers of 10 leave n times the rounding unit and a factor."""
+    rng = np.random.default_rng(n)
+    K = 2
+    A, info = mx.Matrix(n, K), np.zeros(K, np.int32)
+    q = [np.linalg.qr(cv(rng, n, n))[0] for _ in range(K)]
+    a = np.array([(u * np.linspace(1.0, 10.0, n)) @ u.conj().T for u in q])
+    a = (a + np.conj(np.transpose(a, (0, 2, 1)))) / 2
+    A.put(a)
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    assert not info.any()
+    assert rel(A.get(), np.linalg.inv(a)) < 100 * n * 2.2e-16
+    a[1] -= 20.0 * np.eye(n)
+    A.put(a)
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    assert info[0] == 0 and info[1] != 0
