@@ -1158,16 +1158,16 @@ extern "C" int mxk_block_gram(int n, int m, int K, const double* ph, mxk_kappa k
   for (int q = 1; q < nb; q++) lo_rest = lo_rest && precs[q] == MX_C64;
   if (hi_dd && lo_rest && m <= 16 && nb <= 3 && (nb == 1 || resid)) {
     size_t sm = gram_split_smem();
-    cudaFuncSetAttribute(k_block_gram_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+    allow_smem(k_block_gram_split);
     k_block_gram_split<<<dim3(a.chunks, K, nb > 1 ? 2 : 1), GS_T, sm, st>>>(a);
   } else if (hi_dd) {
-    cudaFuncSetAttribute(k_block_gram<dd, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_block_gram<dd, false>);
     for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<dd, false><<<g, GT, smem, st>>>(a, mh, eb);
   } else if (all128) {
-    cudaFuncSetAttribute(k_block_gram<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_block_gram<double, true>);
     for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, true><<<g, GT, smem, st>>>(a, mh, eb);
   } else {
-    cudaFuncSetAttribute(k_block_gram<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_block_gram<double, false>);
     for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, false><<<g, GT, smem, st>>>(a, mh, eb);
   }
   MX_CHECK_LAUNCH();
@@ -1210,10 +1210,10 @@ extern "C" int mxk_block_combine(int n, int m, int K, int nb, const int* precs, 
     dim3 g2(gx, K);
     size_t sm = combine_tiled_smem();
     if (pout == MX_CDD) {
-      cudaFuncSetAttribute(k_block_combine_tiled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+      allow_smem(k_block_combine_tiled<true>);
       k_block_combine_tiled<true><<<g2, CT, sm, st>>>(a, out);
     } else {
-      cudaFuncSetAttribute(k_block_combine_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+      allow_smem(k_block_combine_tiled<false>);
       k_block_combine_tiled<false><<<g2, CT, sm, st>>>(a, out);
     }
     MX_CHECK_LAUNCH();
@@ -1233,7 +1233,7 @@ extern "C" int mxk_block_combine(int n, int m, int K, int nb, const int* precs, 
 #define MX_CB(SO, RO, DD)                                                                                             \
   do {                                                                                                                \
     const size_t sm = ncoef * (sizeof(cx<RO>) + sizeof(cx<float>));                                                   \
-    cudaFuncSetAttribute(k_block_combine<SO, RO, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);          \
+    allow_smem(k_block_combine<SO, RO, DD>);          \
     k_block_combine<SO, RO, DD><<<g, b, sm, st>>>(a, (SO*) out);                                                      \
   } while (0)
   if (pout == MX_CDD) { if (hidd) MX_CB(cdd, dd, true); else MX_CB(cdd, dd, false); }

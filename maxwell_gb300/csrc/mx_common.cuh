@@ -315,6 +315,16 @@ __device__ __forceinline__ dd warp_sum(dd v) {
   return v;
 }
 
+// Lets a kernel take more dynamic shared memory than the default 48 KB: up to
+// SMEM_MOST, the 227 KB of a CTA less 1 KB for static variables.  The limit
+// belongs to the kernel and all threads of the process share it, so it is one
+// value and never the size of the call at hand, which a thread with a smaller
+// call could put in its place between another thread's setting and launch.
+constexpr int SMEM_MOST = 226 * 1024;
+template <typename F> inline void allow_smem(F* kern) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST);
+}
+
 }  // namespace mx
 
 #define MX_CHECK_LAUNCH() do { cudaError_t e_ = cudaGetLastError(); if (e_ != cudaSuccess) return (int) e_; } while (0)

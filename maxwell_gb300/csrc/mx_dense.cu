@@ -632,7 +632,7 @@ size_t jacobi_smem(int N) {
 extern "C" int mxk_hpd_inverse(int N, int K, double* a, int* info, mx_stream s) {
   const size_t smem = sweep_smem(N);
   if (smem <= 208 * 1024) {   // orders up to 160
-    cudaFuncSetAttribute(k_hpd_inverse_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_hpd_inverse_sweep);
     k_hpd_inverse_sweep<<<K, SWT, smem, (cudaStream_t) s>>>(N, a, info);
   } else {
     k_hpd_inverse<<<K, DT, 2 * N * sizeof(Z), (cudaStream_t) s>>>(N, a, info);
@@ -675,7 +675,7 @@ extern "C" int mxk_rayleigh_ritz(int ns, int m, int K, const double* ga, const d
   int in_smem = ns <= 48;
   if (in_smem) {
     smem += 16 + sizeof(double) * 2 * (size_t) ritz_ld(ns) * ns * 5;
-    cudaFuncSetAttribute(k_rayleigh_ritz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_rayleigh_ritz);
   }
   int threads = in_smem ? 512 : 1024;
   k_rayleigh_ritz<<<K, threads, smem, (cudaStream_t) s>>>(ns, m, ga, gm, sel, drop, theta_min, coef, theta, info,
@@ -789,10 +789,10 @@ extern "C" int mxk_coarse_pairs(int n, int m, int K, const double* ph, const dou
   const size_t smem = sizeof(double) * (4 * half + 32 + 2 * nc + 4 * n + (in_smem ? (size_t) 6 * ritz_ld(nc) * nc : 0))
                       + sizeof(int) * 2 * half;
   if (prec_e == MX_CDD) {
-    cudaFuncSetAttribute(k_coarse_pairs<cdd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_coarse_pairs<cdd>);
     k_coarse_pairs<cdd><<<K, 512, smem, (cudaStream_t) s>>>(n, m, K, ph, kappa, work, in_smem, (cdd*) E, mu, info);
   } else if (prec_e == MX_C128) {
-    cudaFuncSetAttribute(k_coarse_pairs<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    allow_smem(k_coarse_pairs<double2>);
     k_coarse_pairs<double2><<<K, 512, smem, (cudaStream_t) s>>>(n, m, K, ph, kappa, work, in_smem, (double2*) E, mu,
                                                                 info);
   } else return (int) cudaErrorInvalidValue;
@@ -857,7 +857,7 @@ __global__ void k_chol_qr_coef(int m, const double* __restrict__ gm, double* __r
 extern "C" int mxk_chol_qr_coef(int m, int K, const double* gm, double* coef, int* info, mx_stream s) {
   if (m < 1 || m > 64) return (int) cudaErrorInvalidValue;
   size_t smem = sizeof(double) * 2 * (size_t) m * m;
-  cudaFuncSetAttribute(k_chol_qr_coef, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  allow_smem(k_chol_qr_coef);
   k_chol_qr_coef<<<K, 64, smem, (cudaStream_t) s>>>(m, gm, coef, info);
   MX_CHECK_LAUNCH();
   return 0;

@@ -746,7 +746,7 @@ int run(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
   auto kern = k_node_vcycle<S, R, MS, false>;
   if constexpr (std::is_same<R, double>::value)
     if (cl > 1) kern = k_node_vcycle<S, R, MS, true>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  allow_smem(kern);
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = cl;
@@ -796,7 +796,7 @@ extern "C" int mxk_node_band_pre(int n, int m, int K, int nu, const double* ph, 
                                  void* bc, mx_stream s) {
   const int halo = 4 * nu + 3, B = band_rows(n, K * m, halo), nb = (n + B - 1) / B;
   const size_t smem = (size_t) (B + halo) * ((n + 127) / 128 * 128) * sizeof(float2);
-  cudaFuncSetAttribute(k_node_band<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  allow_smem(k_node_band<false>);
   k_node_band<false><<<(unsigned) nb * K * m, NBT, smem, (cudaStream_t) s>>>(
       n, m, K, B, nu, ph, (float) (1.0 / 3.0), (const float2*) b, (const float2*) xin, nullptr, (float2*) xout, (float2*) bc);
   MX_CHECK_LAUNCH();
@@ -807,7 +807,7 @@ extern "C" int mxk_node_band_post(int n, int m, int K, int nu, const double* ph,
                                   const void* xc, void* xout, mx_stream s) {
   const int halo = 4 * nu, B = band_rows(n, K * m, halo), nb = (n + B - 1) / B;
   const size_t smem = (size_t) (B + halo) * ((n + 127) / 128 * 128) * sizeof(float2);
-  cudaFuncSetAttribute(k_node_band<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  allow_smem(k_node_band<true>);
   k_node_band<true><<<(unsigned) nb * K * m, NBT, smem, (cudaStream_t) s>>>(
       n, m, K, B, nu, ph, (float) (1.0 / 3.0), (const float2*) b, (const float2*) xin, (const float2*) xc, (float2*) xout,
       nullptr);

@@ -350,8 +350,7 @@ int run_sweep(int n, int m, int K, const double* ph, double alpha, int bwd, int 
   const size_t BS = (size_t) TT::W * VB * sizeof(S);
   const unsigned gx = (unsigned) (a.G * (n / T));
   const size_t tile_smem = (size_t) (2 * P + 3 + 2 * (P + 1) + 3) * BS;
-  cudaFuncSetAttribute(k_node_gs_tile<S, R, D, VB, RL, T, NTH, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int) tile_smem);
+  allow_smem(k_node_gs_tile<S, R, D, VB, RL, T, NTH, P>);
   k_node_gs_single<S, R, D, VB, RL, T, NTH><<<dim3(gx, 1, K), NTH, 5 * BS, st>>>(a);
   MX_CHECK_LAUNCH();
   const int Q = (n - 2) / 2;

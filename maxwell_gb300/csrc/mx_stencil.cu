@@ -1854,7 +1854,7 @@ static int L_edge_gs_rows(int n, int m, int K, const double* ph, mxk_kappa kap, 
   if (threads < ((8 * VB + 31) & ~31)) threads = (8 * VB + 31) & ~31;
   const int SEG = n < 256 ? n : 256;
   const size_t smem = sizeof(R) * ((size_t) (P + 1) * VB * 14 + (size_t) SEG * 28);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_edge_gs_scan<S, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  if (smem > 48 * 1024) allow_smem(k_edge_gs_scan<S, R>);
   k_edge_gs_scan<S, R><<<dim3((unsigned) rows * K, (m + VB - 1) / VB), threads, smem, st>>>(
       n, m, K, ph, make_kap<R>(kap, n), axy, mm, s8, is8, j0, VB, P, SEG, backward, (const S*) b, (S*) x);
   MX_CHECK_LAUNCH();
@@ -1899,7 +1899,7 @@ static int L_node_gs_rows_d(int n, int m, int K, const double* ph, double alpha,
     const size_t smem = (size_t) (full + 1) * m * sizeof(cx<R>);
     if (m <= 32 && smem <= 96 * 1024 && nrows == 1) {
       if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_node_gs_rowpar<S, R, D, LR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        allow_smem(k_node_gs_rowpar<S, R, D, LR>);
       k_node_gs_rowpar<S, R, D, LR><<<dim3(nrows, K), blk2(m), smem, st>>>(n, m, K, ph, inv_ac, third, j0, jstep,
                                                                            backward, full - 1, (const S*) b, (S*) x);
       MX_CHECK_LAUNCH();
@@ -1912,7 +1912,7 @@ static int L_node_gs_rows_d(int n, int m, int K, const double* ph, double alpha,
     while (ring < 2 * (int) b2.y * LR + D) ring <<= 1;
     size_t smem = (size_t) (ring + 1) * m * sizeof(cx<R>);
     if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_node_gs_row<S, R, D, LR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+      allow_smem(k_node_gs_row<S, R, D, LR>);
     k_node_gs_row<S, R, D, LR><<<g, b2, smem, st>>>(n, m, K, ph, inv_ac, third, j0, jstep, backward, ring - 1,
                                                      (const S*) b, (S*) x);
   } else {
@@ -1920,7 +1920,7 @@ static int L_node_gs_rows_d(int n, int m, int K, const double* ph, double alpha,
     while (ring < (32 / m) * LR + D) ring <<= 1;
     size_t smem = (size_t) 8 * (ring + 1) * m * sizeof(cx<R>);
     if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_node_gs_warp<S, R, D, LR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+      allow_smem(k_node_gs_warp<S, R, D, LR>);
     k_node_gs_warp<S, R, D, LR><<<dim3((nrows + 7) / 8, K), 256, smem, st>>>(
         n, m, K, ph, inv_ac, third, j0, jstep, nrows, backward, ring - 1, (const S*) b, (S*) x);
   }
