@@ -106,8 +106,11 @@ int mxk_node_rr_get_strips(void);
 /* whole V-cycles of the levels n0 .. n0 << top (nu sweeps each way, the
  * coarse inverse ainv) in one launch: `cycles` of them on b, x of the top
  * level, x starting from zero where zero is set.  mxk_node_vcycle_top: the
- * highest level up to `top` that this form takes (0: none) */
+ * highest level up to `top` that this form takes (0: none);
+ * mxk_node_vcycle_pays: whether it is the faster form for a batch of vecs
+ * vectors when no level above takes bands */
 int mxk_node_vcycle_top(int n0, int top, int prec);
+int mxk_node_vcycle_pays(int vecs, int prec);
 int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
                     const double *phases, const double *ainv, const void *ainv_c64, int prec,
                     const void *b, void *x, mx_stream s);

@@ -765,14 +765,29 @@ int run(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
 }  // namespace
 
 // Every level whose chain of levels fits into a CTA's shared memory, up to 96
-// nodes a side (three positions per lane): c64 64 and 96, FP64 64.  Measured
-// as above for 64; with 1 to 512 vectors in the batch the launches it
-// replaces cost more.  The coarse solve wants n0^2 <= NCT / 2 rows.
+// nodes a side (three positions per lane): c64 64 and 96, FP64 64.  The coarse
+// solve wants n0^2 <= NCT / 2 rows.
 extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
   if (n0 < 4 || (n0 & 1) || n0 > 16) return 0;
   int l = 0;
   while (l < top && (n0 << (l + 1)) <= 96 && cycle_smem(n0, l + 1, prec) <= 200 * 1024) l++;
   return l;
+}
+
+// A CTA per vector: past the batch that the SMs hold at once the launch takes a
+// multiple of its time, while the row kernels it replaces only then begin to
+// fill the GPU.  One launch against theirs, cycles from 16 and 32 to 4 or 8,
+// from 64, 80 and 96 to 8, 10 and 12 and from 32 and 64 to 16, ms:
+// c64    2048 vectors 0.21/0.22 .. 1.60/1.71 (all between 0.80 and 0.97),
+//        4096 vectors 0.64/0.40 and 0.97/0.70 (16, 32), 1.46/1.43 (64)
+// FP64   1024 vectors 0.53/0.64 .. 7.2/7.6, 2048 vectors 1.78/1.03 and
+//        3.30/2.55 (16, 32), 6.97/7.02 (64)
+// cdd    448 vectors 0.32/0.39 .. 2.37/2.45, 768 vectors 0.58/0.40 and
+//        1.06/0.86 (16, 32), 1.99/1.96 (64), 3.40/2.78 (96)
+// (Under a level that takes bands the launch serves every batch: the bands'
+// planar vectors need it, and they gain more than it loses.)
+extern "C" int mxk_node_vcycle_pays(int vecs, int prec) {
+  return vecs <= (prec == MX_C64 ? 2048 : prec == MX_C128 ? 1024 : 448);
 }
 
 extern "C" int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,

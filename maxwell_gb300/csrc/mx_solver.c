@@ -474,6 +474,13 @@ static int fused_node_cycles(mxg_solver *s, int l, int cycles, int zero, int pla
   return 0;
 }
 
+/* the highest level up to top that runs in one launch with those below it
+ * where no band kernel takes the levels above (0: none) */
+static int fused_level(const mxg_solver *s, int top)
+{
+  return mxk_node_vcycle_pays(s->K * s->m, s->pg) ? mxk_node_vcycle_top(s->n0, top, s->pg) : 0;
+}
+
 /* The lifting of level l runs on planar vectors when every level of its node
  * V-cycle has a kernel of that form: the bands of the fine levels, one launch
  * for the rest (the opt-in tiled sweep keeps its own layout).  Decided when
@@ -483,7 +490,7 @@ static int planar_level(const mxg_solver *s, int l)
   int lc, q;
   if(s->pg != MX_C64 || mxk_node_gs_oop_ok(s->n[l], s->m, s->pg)) return 0;
   lc = mxk_node_vcycle_top(s->n0, l, s->pg);
-  if(lc == 0) return 0;
+  if(lc == 0 || (lc == l && fused_level(s, l) == 0)) return 0;
   for(q = lc + 1; q <= l; q++)
     if(!mxk_node_band_ok(s->n[q], s->m, s->o.smoother_steps, s->pg)) return 0;
   return 1;
@@ -513,7 +520,7 @@ static int vcycle_n_planar(mxg_solver *s, int top, int zero)
 /* vcycle_node2d (node2d.c:1352-1389) on bg[top], xg[top] */
 static int vcycle_n(mxg_solver *s, int top)
 {
-  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg, lc = mxk_node_vcycle_top(s->n0, top, pg);
+  int l, nu = s->o.smoother_steps, m = s->m, K = s->K, pg = s->pg, lc = fused_level(s, top);
   for(l = top; l > lc; l--) {
     int n = s->n[l];
     TRY(node_smooth(s, l, 0, nu));
@@ -573,7 +580,7 @@ static int run_graphed(mxg_solver *s, int l, cudaGraphExec_t *exec, long *nlaunc
 static int lift_body(mxg_solver *s, int l)
 {
   int i;
-  if(l > 0 && mxk_node_vcycle_top(s->n0, l, s->pg) == l)
+  if(l > 0 && fused_level(s, l) == l)
     return fused_node_cycles(s, l, s->o.gradient_steps, 1, s->planar[l]);
   if(s->planar[l]) {
     for(i = 0; i < s->o.gradient_steps; i++)

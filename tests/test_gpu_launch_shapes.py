@@ -271,3 +271,94 @@ def test_hermitian_inverse_orders(n):
     A.put(a)
     mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
     assert info[0] == 0 and info[1] != 0
+
+
+def node_levels(n0, L, K, m, prec, fac):
+    """Grids, b, x, d of a node hierarchy (coarsest first), the factored
+    coarse matrix and the handles' arrays."""
+    import ctypes as C
+    grids = [mx.Grid(n0 << L, K, None, fac)]
+    for _ in range(L):
+        grids.append(grids[-1].coarsen())
+    grids = grids[::-1]
+    b, x, d = ([mx.Node(g, m, prec) for g in grids] for _ in range(3))
+    A, info = mx.Matrix(n0 * n0, K), np.zeros(K, np.int32)
+    mx.check(mx.lib().densematrix_node2d_gpu(1, grids[0].h, A.h))
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    return b, x, d, A, [(C.c_void_p * (L + 1))(*[o.h for o in objs]) for objs in (b, x, d)]
+
+
+def node_cycle(oracle, n0, l, f, b, x, nu=2):
+    """A V-cycle of one vector put together from the oracle's sweeps,
+    residual and transfers."""
+    n = n0 << l
+    if l == 0:
+        return np.linalg.solve(oracle.dense_node(n0, *f, 1), b)
+    for _ in range(nu):
+        x = oracle.gs_node(n, *f, 1.0, 0, b, x)
+    r = oracle.addeval_node(n, *f, -1.0, x, b)
+    c = oracle.restrict_node(n // 2, *f, 1.0, r, np.zeros(n * n // 4, complex))
+    x = oracle.prolong_node(n // 2, *f, 1.0, node_cycle(oracle, n0, l - 1, f, c, np.zeros_like(c), nu), x)
+    for _ in range(nu):
+        x = oracle.gs_node(n, *f, 1.0, 1, b, x)
+    return x
+
+
+@pytest.mark.parametrize("prec, K", [(mx.C64, 65), (mx.C128, 33), (mx.CDD, 15)])
+def test_node_vcycle_large_batch(oracle, prec, K):
+    """Coarse node levels of batches of more vectors than the one-launch form
+    takes, which run level by level."""
+    n0, L, m = 4, 2, 32
+    n = n0 << L
+    rng = np.random.default_rng(K)
+    fac = np.exp(1j * rng.uniform(0.3, 3.0, (K, 2)))
+    b, x, d, A, arr = node_levels(n0, L, K, m, prec, fac)
+    b[L].put(cv(rng, K, m, n * n))
+    x[L].put(cv(rng, K, m, n * n))
+    rhs, start = b[L].get(), x[L].get()
+    mx.check(mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr))
+    got = x[L].get()
+    for k, v in [(0, 0), (K // 2, m // 2), (K - 1, m - 1)]:
+        want = node_cycle(oracle, n0, L, fac[k], rhs[k, v], start[k, v])
+        assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 1e-10)
+
+
+@pytest.mark.parametrize("prec, n0, L, K, m", [(mx.C64, 8, 1, 512, 32), (mx.C128, 8, 1, 512, 32), (mx.CDD, 8, 2, 256, 32)])
+def test_node_vcycle_large_batch_costs_its_sweeps(prec, n0, L, K, m):
+    """A V-cycle of a large batch takes no longer than the sweeps, residuals,
+    transfers and coarse solve it stands for, called one by one (with half as much again
+    for the timing; one CTA per vector took 2.3 to 4.5 times as long)."""
+    import time
+    lib, one = mx.lib(), mx.fz(1.0)
+    b, x, d, A, arr = node_levels(n0, L, K, m, prec, np.exp(1j * np.random.default_rng(1).uniform(0.3, 3.0, (K, 2))))
+    mx.check(lib.random_node2d_gpu(b[L].h, 3))
+    mx.check(lib.zero_node2d_gpu(x[L].h))
+
+    def whole():
+        mx.check(lib.vcycle_node2d_gpu(L, 2, A.h, *arr))
+
+    def parts():
+        for l in range(L, 0, -1):
+            for _ in range(2):
+                mx.check(lib.gsforward_node2d_gpu(one, b[l].h, x[l].h))
+            mx.check(lib.copy_node2d_gpu(b[l].h, d[l].h))
+            mx.check(lib.addeval_node2d_gpu(mx.fz(-1.0), x[l].h, d[l].h))
+            mx.check(lib.zero_node2d_gpu(b[l - 1].h))
+            mx.check(lib.restriction_node2d_gpu(one, d[l].h, b[l - 1].h))
+            mx.check(lib.zero_node2d_gpu(x[l - 1].h))
+        mx.check(lib.vcycle_node2d_gpu(0, 2, A.h, *arr))   # the coarse solve
+        for l in range(1, L + 1):
+            mx.check(lib.prolongation_node2d_gpu(one, x[l - 1].h, x[l].h))
+            for _ in range(2):
+                mx.check(lib.gsbackward_node2d_gpu(one, b[l].h, x[l].h))
+
+    def seconds(f):
+        f()
+        times = []
+        for _ in range(5):
+            t = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t)
+        return sorted(times)[2]
+
+    assert seconds(whole) < 1.5 * seconds(parts)
