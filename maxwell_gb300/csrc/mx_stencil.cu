@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 using namespace mx;
 
@@ -536,21 +537,29 @@ __device__ void afw_patch_matrices(R kLL, R kUL, R kLR, R kUR, R axy, R mm, R s8
   }
 }
 
-template <typename S, typename R>
+//
+// FLAT: a CTA's VB vectors are any VB of the batch's (k-point, vector) pairs,
+// not vectors of one k-point: the matrices do not depend on k, and a CTA of one
+// or two vectors pays the row's matrices and a warp's recurrence for them
+// alone.  c128, one vector at each of 32 k-points, 256^2 2.31 -> 1.02 ms; at
+// 2048 k-points, 16^2 1.40 -> 0.34 ms.
+template <typename S, typename R, bool FLAT>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_edge_gs_scan(int n, int m, int K, const double* __restrict__ ph, Kap<R> kap,
                                                       Sc axy_s, Sc mm_s, Sc s8_s, Sc is8_s, int j0, int VB, int P,
                                                       int SEG, int backward, const S* __restrict__ b, S* x) {
-  // grid (rows of the phase x K, groups of VB vectors); column c = tid / VB
-  // of the chunk, 0 the one before it; P patches per chunk
+  // grid (rows of the phase x K, groups of VB vectors), FLAT (rows of the
+  // phase x groups of VB pairs); column c = tid / VB of the chunk, 0 the one
+  // before it; P patches per chunk
   extern __shared__ __align__(16) unsigned char smem_rows[];
   R* D = reinterpret_cast<R*>(smem_rows);              // [P + 1][VB][2][4] corrections
   cx<R>* W = reinterpret_cast<cx<R>*>(D + (P + 1) * VB * 8);   // [P + 1][3][VB] curls, x residual
   R* Sm = reinterpret_cast<R*>(W + (P + 1) * VB * 3);  // [SEG][16]
   R* Tm = Sm + SEG * 16;                               // [SEG][12]
-  const int tid = threadIdx.x, rows = n / 2, k = blockIdx.x / rows, v0 = blockIdx.y * VB;
-  const int j = j0 + 2 * (int) (blockIdx.x - k * rows);
-  const int c = tid / VB, vv = tid - c * VB, v = v0 + vv < m ? v0 + vv : m - 1;
-  const bool live = v0 + vv < m;
+  const int tid = threadIdx.x, rows = n / 2, kb = blockIdx.x / rows;
+  const int j = j0 + 2 * (int) (blockIdx.x - kb * rows);
+  const int c = tid / VB, vv = tid - c * VB, at = (FLAT ? kb : (int) blockIdx.y) * VB + vv;
+  const bool live = at < (FLAT ? K * m : m);
+  const int k = !FLAT ? kb : live ? at / m : K - 1, v = !live ? m - 1 : FLAT ? at - k * m : at;
   Lay L{n, m, K};
   const Seam<R> seam = seam_load<R>(ph, K, k, n);
   S* xk = x + L.edge(k, 0, 0, 0, v);
@@ -1826,7 +1835,10 @@ extern "C" size_t mxk_elem_size(int prec) { return prec == MX_C64 ? 8 : 16; }
 // are enough chains to hide its latency: forward sweep of 16 vectors, chain
 // against recurrence, 0.55 / 0.40 ms at 32768 chains (128^2, 32 k-points),
 // 2.09 / 1.40 (512^2, 8), 2.18 / 2.02 at 49152 (512^2, 12), 1.15 / 1.37 at
-// 65536 (256^2, 32), 2.30 / 2.63 (512^2, 16).
+// 65536 (256^2, 32), 2.30 / 2.63 (512^2, 16).  On grids up to 64^2 it would
+// from some 2048 vectors on (16^2, 4096 vectors 0.046 / 0.069, 32^2, 2048
+// 0.083 / 0.116); the recurrence stays there for its rounding, which does not
+// grow with n^2 (error of a sweep at 32^2 6e-7 against 6e-5).
 template <typename S, typename R>
 static int L_edge_gs_rows(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,
                           double beta, int j0, int backward, const void* b, void* x, cudaStream_t st) {
@@ -1844,19 +1856,41 @@ static int L_edge_gs_rows(int n, int m, int K, const double* ph, mxk_kappa kap, 
       return 0;
     }
   }
-  // a CTA takes VB vectors of a row: all of them, or as few as four where
-  // rows x k-points leave SMs without a CTA
+  // a CTA takes VB vectors of a row: all of a k-point's, or as few as four
+  // where rows x k-points leave SMs without a CTA
   int VB = m;
   while (VB > 4 && (size_t) rows * K * ((m + VB - 1) / VB) < 2 * 152) VB = (VB + 1) / 2;
+  // Vectors of several k-points in a CTA where there are CTAs to spare, by
+  // measurement (forward sweeps, ms, one k-point a CTA / several).  FP64 and
+  // float-float: one or two vectors (c128 64^2, 32 k-points of one 0.21 /
+  // 0.13); below eight up to 128^2, float-float in larger batches (c128 64^2,
+  // 32 k-points of five 0.52 / 0.42, 48^2 0.30 / 0.33; 256^2, 8 k-points 1.31 /
+  // 1.37; cdd 64^2, 32 k-points of three 0.14 / 0.16); small grids of many
+  // k-points (c128 64^2 x 16, 128 k-points 3.38 / 2.81, 32 k-points 0.95 /
+  // 0.98).  c64: one vector (256^2, 8 k-points 0.101 / 0.072), two in large
+  // batches (128^2, 128 k-points 0.50 / 0.33; 16 k-points 0.068 / 0.076).
+  const size_t ctas = (size_t) rows * K * ((m + VB - 1) / VB);
+  constexpr bool f64 = std::is_same<R, double>::value;
+  bool flat;
+  if (sizeof(R) == 4) flat = m == 1 ? ctas >= 1024 : m == 2 && ctas >= 4096;
+  else if (m <= 2) flat = ctas > 4 * 152;
+  else if (m < 8) flat = n <= 128 && ctas >= (!f64 ? 4096 : n <= 16 ? 2048 : 1024);
+  else flat = m < 32 && n <= 64 && ctas >= (f64 && n <= 16 ? 1024 : 2048);
+  if (flat) {
+    VB = std::min(K * m, sizeof(R) == 4 ? 16 : 32);
+    while (VB > 4 && (size_t) rows * ((K * m + VB - 1) / VB) < 2 * 152) VB = (VB + 1) / 2;
+  }
   int P = 256 / VB - 1;
   if (P > n / 2) P = n / 2;
   int threads = ((P + 1) * VB + 31) & ~31;
   if (threads < ((8 * VB + 31) & ~31)) threads = (8 * VB + 31) & ~31;
   const int SEG = n < 256 ? n : 256;
   const size_t smem = sizeof(R) * ((size_t) (P + 1) * VB * 14 + (size_t) SEG * 28);
-  if (smem > 48 * 1024) allow_smem(k_edge_gs_scan<S, R>);
-  k_edge_gs_scan<S, R><<<dim3((unsigned) rows * K, (m + VB - 1) / VB), threads, smem, st>>>(
-      n, m, K, ph, make_kap<R>(kap, n), axy, mm, s8, is8, j0, VB, P, SEG, backward, (const S*) b, (S*) x);
+  auto kern = flat ? k_edge_gs_scan<S, R, true> : k_edge_gs_scan<S, R, false>;
+  if (smem > 48 * 1024) allow_smem(kern);
+  const dim3 grid = flat ? dim3((unsigned) rows * ((K * m + VB - 1) / VB)) : dim3((unsigned) rows * K, (m + VB - 1) / VB);
+  kern<<<grid, threads, smem, st>>>(n, m, K, ph, make_kap<R>(kap, n), axy, mm, s8, is8, j0, VB, P, SEG, backward,
+                                    (const S*) b, (S*) x);
   MX_CHECK_LAUNCH();
   return 0;
 }

@@ -362,3 +362,76 @@ def test_node_vcycle_large_batch_costs_its_sweeps(prec, n0, L, K, m):
         return sorted(times)[2]
 
     assert seconds(whole) < 1.5 * seconds(parts)
+
+
+@pytest.mark.parametrize("prec, n, m, K", [(mx.C64, 16, 1, 200), (mx.C64, 64, 2, 150),
+                                           (mx.C128, 8, 1, 1100), (mx.C128, 64, 2, 20), (mx.C128, 4, 16, 520),
+                                           (mx.C128, 130, 1, 21), (mx.C128, 2, 1, 2500), (mx.CDD, 8, 5, 1030),
+                                           (mx.CDD, 32, 1, 1100), (mx.CDD, 64, 3, 130)])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_row_smoother_pairs(oracle, prec, n, m, K, direction):
+    """The patch smoother in row order where a CTA takes vectors of several
+    k-points (few vectors of many k-points, small grids), groups that the
+    batch does not fill, and the smallest grid in a c64 batch that would be
+    large enough for a thread per chain."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(0.3, 3.0, (K, 2)))
+    g = mx.Grid(n, K, kap, fac)
+    b, x = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    eb, ex = mx.Edge(g, m, prec, b), mx.Edge(g, m, prec, x)
+    fn = [mx.lib().gsforward_edge2d_gpu, mx.lib().gsbackward_edge2d_gpu][direction]
+    mx.check(fn(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h))
+    got = ex.get()
+    for k in {0, 1, K // 2, K - 2, K - 1}:
+        for v in {0, m - 1}:
+            want = oracle.gs_edge(n, kap, *fac[k], 1.0, 0.8, direction, b[k, v], x[k, v])
+            assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 1e-11)
+
+
+@pytest.mark.parametrize("beta", [1.0, 0.8])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_row_smoother_chains(oracle, beta, direction):
+    """The c64 patch smoother in row order with a thread per row and vector
+    (57344 chains and more), with the scalars that the tabulated factors were
+    made for and with others.  Its residuals are differences of curls of size
+    n^2 rounded to 2^-24, four to an edge, which the local solve does not
+    divide by n^2 again in the direction of the vertex' gradient."""
+    n, m, K = 128, 32, 28
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(0.3, 3.0, (K, 2)))
+    g = mx.Grid(n, K, kap, fac)
+    b, x = cv(rng, 1, m, 2 * n * n), cv(rng, 1, m, 2 * n * n)   # the same block at every k-point
+    eb, ex = mx.Edge(g, m, mx.C64, b), mx.Edge(g, m, mx.C64, x)
+    fn = [mx.lib().gsforward_edge2d_gpu, mx.lib().gsbackward_edge2d_gpu][direction]
+    mx.check(fn(mx.fz(1.0), mx.fz(beta), eb.h, ex.h))
+    got = ex.get()
+    for k, v in {(0, 0), (K // 2, m // 2), (K - 1, m - 1)}:
+        want = oracle.gs_edge(n, kap, *fac[k], 1.0, beta, direction, b[0, v], x[0, v])
+        assert rel(got[k, v], want) < 4 * n * n * 2.0 ** -24
+
+
+@pytest.mark.parametrize("prec, n", [(mx.C128, 16), (mx.CDD, 32)])
+def test_row_smoother_batch_shape(prec, n):
+    """The row-order smoother costs about as much for a vector at each of
+    2048 k-points as for 32 at 64 (2.4 to 4.3 times as much where a CTA held
+    vectors of one k-point only)."""
+    import time
+    lib, one, dot = mx.lib(), mx.fz(1.0), np.zeros(2048)
+    times = []
+    for K, m in ((2048, 1), (64, 32)):
+        g = mx.Grid(n, K, np.full(n * n, 0.5), np.exp(1j * np.random.default_rng(1).uniform(0.3, 3.0, (K, 2))))
+        b, x = mx.Edge(g, m, prec), mx.Edge(g, m, prec)
+        mx.check(lib.random_edge2d_gpu(b.h, 3))
+        mx.check(lib.zero_edge2d_gpu(x.h))
+        runs = []
+        for _ in range(6):
+            mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))   # waits
+            t = time.perf_counter()
+            for _ in range(10):
+                mx.check(lib.gsforward_edge2d_gpu(one, one, b.h, x.h))
+            mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))
+            runs.append(time.perf_counter() - t)
+        times.append(sorted(runs[1:])[2])
+    assert times[0] < 1.7 * times[1]
