@@ -1847,7 +1847,7 @@ static int L_edge_gs_rows(int n, int m, int K, const double* ph, mxk_kappa kap, 
            is8 = make_sc(6.0 / (8.0 * beta));
   const size_t chains = (size_t) rows * m * K;
   if constexpr (sizeof(R) == 4) {
-    if (chains >= 57344) {
+    if (chains >= 57344 && n >= 4) {   // (it reads a column ahead, which at n = 2 is its own)
       // the tabulated factors serve the scalars they were made for
       const float4* ftab = (kap.afw && kap.afw_alpha == alpha && kap.afw_beta == beta) ? (const float4*) kap.afw : nullptr;
       k_edge_gs_rows<S, R><<<nblocks(chains, 64), 64, 0, st>>>(n, m, K, ph, make_kap<R>(kap, n), ftab, axy, mm, s8, is8,

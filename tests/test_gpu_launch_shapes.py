@@ -364,7 +364,7 @@ def test_node_vcycle_large_batch_costs_its_sweeps(prec, n0, L, K, m):
     assert seconds(whole) < 1.5 * seconds(parts)
 
 
-@pytest.mark.parametrize("prec, n, m, K", [(mx.C64, 16, 1, 200), (mx.C64, 64, 2, 150),
+@pytest.mark.parametrize("prec, n, m, K", [(mx.C64, 16, 1, 200), (mx.C64, 64, 2, 150), (mx.C64, 2, 32, 1800),
                                            (mx.C128, 8, 1, 1100), (mx.C128, 64, 2, 20), (mx.C128, 4, 16, 520),
                                            (mx.C128, 130, 1, 21), (mx.C128, 2, 1, 2500), (mx.CDD, 8, 5, 1030),
                                            (mx.CDD, 32, 1, 1100), (mx.CDD, 64, 3, 130)])
