@@ -844,7 +844,7 @@ template <typename R> struct alignas(16) AfwSlot {
   R l20, l21, i0, i1, i2, pad[3];
 };
 constexpr int AFW_TAB_BYTES = 48 * 1024;   // most shared memory that a CTA's table of patches takes
-constexpr int AFW_PARTS = 4;               // CTAs that share a row
+constexpr int AFW_PARTS = 4;               // CTAs that share a row that is cut
 
 // afw_patch with the weights and factors from a table
 template <typename S, typename R>
@@ -2126,7 +2126,20 @@ template <typename S, typename R>
 static int L_edge_gs_rowpair(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha, double beta,
                              int cj, int rev, const void* b, void* x, cudaStream_t st) {
   if constexpr (sizeof(S) > 8) {
-    const int h = n / 2, nseg = h >= AFW_PARTS ? AFW_PARTS : 1, part = (h + nseg - 1) / nseg;
+    // Rows are cut over a cluster unless there are rows enough: a CTA of a
+    // whole row fills its warps better and makes each patch's factors once.
+    // Sweeps of FP64 (f) and float-float (d) blocks, cut / whole, ms: 8^2 x 16
+    // at 512 k-points f 0.66 / 0.34, d 1.46 / 0.26; 64^2 x 6 at 128 d 2.70 /
+    // 1.15 (a row per CTA without the table 2.07), 32^2 x 16 at 64 d 0.47 /
+    // 0.36, f 0.50 / 0.46, at 32 f 0.28 / 0.33; 130^2 x 16 at 32 d 2.88 / 2.27;
+    // 64^2 x 16 at 64 d 1.23 / 1.29, f 1.46 / 1.49, at 128 d 2.95 / 2.25, f
+    // 2.81 / 2.73.
+    const int h = n / 2;
+    const size_t rows = (size_t) h * K;
+    const bool whole = h < AFW_PARTS || rows >= 3072 || (m < 8 && n <= 128 && rows >= 512) ||
+                       (n <= 16 && rows >= 384) || (m < 32 && n <= 32 && rows >= 1024) ||
+                       (std::is_same<R, dd>::value && rows >= 1920 && (n > 64 || m > 16));
+    const int nseg = whole ? 1 : AFW_PARTS, part = (h + nseg - 1) / nseg;
     const int pairs = (AFW_TAB_BYTES / (int) sizeof(AfwSlot<R>) - 1) / 2;   // first-colour patches of a table
     const int P = std::min({256 / m, part, pairs}), T = std::min(pairs / P, (part + P - 1) / P);
     cudaLaunchAttribute at;

@@ -435,3 +435,48 @@ def test_row_smoother_batch_shape(prec, n):
             runs.append(time.perf_counter() - t)
         times.append(sorted(runs[1:])[2])
     assert times[0] < 1.7 * times[1]
+
+
+@pytest.mark.parametrize("n, m, K", [(8, 16, 100), (32, 5, 40), (64, 1, 20), (32, 17, 70), (66, 16, 60)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_colour_smoother_whole_rows(oracle, n, m, K, prec, direction):
+    """The patch smoother in four colours in batches of so many rows that a
+    CTA takes a whole one: one chunk and several, several tables."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(0.3, 3.0, (K, 2)))
+    g = mx.Grid(n, K, kap, fac)
+    b, x = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    eb, ex = mx.Edge(g, m, prec, b), mx.Edge(g, m, prec, x)
+    mx.check(mx.lib().gscolour_edge2d_gpu(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h, direction))
+    got = ex.get()
+    for k in {0, K // 2, K - 1}:
+        for v in {0, m // 2, m - 1}:
+            want = oracle.gs_edge_colour(n, kap, *fac[k], 1.0, 0.8, direction, b[k, v], x[k, v])
+            assert rel(got[k, v], want) < 1e-11
+
+
+@pytest.mark.parametrize("n, m, K", [(64, 6, 512), (8, 16, 512)])
+def test_colour_smoother_batch_shape(n, m, K):
+    """The four-colour smoother of float-float blocks costs about as much for
+    vectors spread over many k-points as for the same number at 32 per
+    k-point (1.7 to 5 times as much with every row cut in four)."""
+    import time
+    lib, one, dot = mx.lib(), mx.fz(1.0), np.zeros(K * m)
+    times = []
+    for kk, mm in ((K, m), (K * m // 32, 32)):
+        g = mx.Grid(n, kk, np.full(n * n, 0.5), np.exp(1j * np.random.default_rng(1).uniform(0.3, 3.0, (kk, 2))))
+        b, x = mx.Edge(g, mm, mx.CDD), mx.Edge(g, mm, mx.CDD)
+        mx.check(lib.random_edge2d_gpu(b.h, 3))
+        mx.check(lib.zero_edge2d_gpu(x.h))
+        runs = []
+        for _ in range(6):
+            mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))   # waits
+            t = time.perf_counter()
+            for _ in range(4):
+                mx.check(lib.gscolour_edge2d_gpu(one, one, b.h, x.h, 0))
+            mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))
+            runs.append(time.perf_counter() - t)
+        times.append(sorted(runs[1:])[2])
+    assert times[0] < 2.0 * times[1]
