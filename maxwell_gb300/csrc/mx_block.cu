@@ -278,14 +278,19 @@ template <> struct HiStore<dd> { using T = cdd; };
 template <> struct HiStore<double> { using T = double2; };
 
 // HI = dd for the mixed solver (column block 0 is cdd, the other blocks c64),
-// double for the plain solver.  ALLHI: every column is high (c128 blocks);
-// the FP32 accumulators and staging do not exist then.  FP64 blocks are bound
+// double for the plain solver.  HIGH: which columns are: none (c64 blocks
+// alone), those of block 0, all (c128 blocks); the accumulators and staging of
+// the other kind do not exist in the first and the last case.  FP64 blocks are bound
 // by the FP64 rate: the site's kappa goes into the staged curl of column j
 // (component 5), entries are pure multiply-adds, and the threads without an
 // entry of their own share the sites.  11 c128 vectors, 120^2, 5 k-points:
-// 0.51 -> 0.26 ms.
-template <typename HI, bool ALLHI>
-__global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int ebase) {
+// 0.51 -> 0.26 ms.  Of c64 blocks three CTAs fit an SM, which counts where the
+// k-points make more CTAs than two each hold (64^2 x 32, 48 k-points, through
+// gram_edge2d_gpu: 0.87 ms with two, 0.69 with three).
+enum { NONE_HIGH, FIRST_HIGH, ALL_HIGH };
+template <typename HI, int HIGH>
+__global__ void __launch_bounds__(GT, HIGH == NONE_HIGH ? 3 : 2) k_block_gram(GramArgs a, int mh, int ebase) {
+  constexpr bool ALLHI = HIGH == ALL_HIGH, ALLLO = HIGH == NONE_HIGH;
   int k = blockIdx.y, chunk = blockIdx.x;
   int n = a.n, m = a.m, ns = a.ns;
   int nent = ns * (ns + 1) / 2;
@@ -307,12 +312,12 @@ __global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int eb
   const int ngr = nent < GT ? (GT / nent < TS ? GT / nent : TS) : 1, gr = ngr > 1 ? (int) threadIdx.x / nent : 0;
   const int et = ngr > 1 ? (int) threadIdx.x - gr * nent : (int) threadIdx.x;
   cx<float> acc_a[ALLHI ? 1 : MAXE], acc_m[ALLHI ? 1 : MAXE];
-  cx<HI> hacc_a[MAXE], hacc_m[MAXE];
+  cx<HI> hacc_a[ALLLO ? 1 : MAXE], hacc_m[ALLLO ? 1 : MAXE];
   int ei[MAXE], ej[MAXE];
 #pragma unroll
   for (int t = 0; t < MAXE; t++) {
     if constexpr (!ALLHI) acc_a[t] = acc_m[t] = czero<float>();
-    hacc_a[t] = czero<HI>(); hacc_m[t] = czero<HI>();
+    if constexpr (!ALLLO) hacc_a[t] = hacc_m[t] = czero<HI>();
     int e = ebase + et + t * GT;
     ei[t] = -1; ej[t] = -1;
     if (e < nent && gr < ngr) {
@@ -339,7 +344,7 @@ __global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int eb
       int prec = a.precs[b];
       size_t o0 = L.edge(k, 0, 0, 0, v);
       cx<float>* ls = lo + ((size_t) ts * ns + col) * 5;
-      if (col < mh) {
+      if (!ALLLO && col < mh) {
         cx<HI> c, x0, y0, mxv, myv;
         // float-float blocks in float-float arithmetic, FP64 blocks in FP64
         using SH = typename HiStore<HI>::T;
@@ -393,17 +398,19 @@ __global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int eb
     for (int t = 0; t < MAXE; t++) {
       int i = ei[t], j = ej[t];
       if (i < 0) continue;
-      if (ALLHI || (i < mh && j < mh)) {
-        cx<HI> sa = czero<HI>(), sm2 = czero<HI>();
-        for (int ts = gr; ts < nts; ts += ngr) {
-          const cx<HI>* hs = hi + (size_t) ts * mh * 6;
-          gram_mac(sa, hs[i * 6], hs[j * 6 + 5]);
-          gram_mac(sm2, hs[i * 6 + 1], hs[j * 6 + 3]);
-          gram_mac(sm2, hs[i * 6 + 2], hs[j * 6 + 4]);
+      if (!ALLLO && (ALLHI || (i < mh && j < mh))) {
+        if constexpr (!ALLLO) {
+          cx<HI> sa = czero<HI>(), sm2 = czero<HI>();
+          for (int ts = gr; ts < nts; ts += ngr) {
+            const cx<HI>* hs = hi + (size_t) ts * mh * 6;
+            gram_mac(sa, hs[i * 6], hs[j * 6 + 5]);
+            gram_mac(sm2, hs[i * 6 + 1], hs[j * 6 + 3]);
+            gram_mac(sm2, hs[i * 6 + 2], hs[j * 6 + 4]);
+          }
+          hacc_a[t] += sa;
+          hacc_m[t] += sm2;
         }
-        hacc_a[t] += sa;
-        hacc_m[t] += sm2;
-      } else if constexpr (!ALLHI) if (use_r && j < mh) {
+      } else if constexpr (!ALLHI) if (!ALLLO && use_r && j < mh) {
         // cross entry s_i^H (A+M) e_j = theta_j s_i^H M e_j + s_i^H r_j: only
         // s_i^H r_j is accumulated here, the rest is added at the end
         cx<float> sa = czero<float>(), sm2 = czero<float>();
@@ -435,8 +442,11 @@ __global__ void __launch_bounds__(GT, 2) k_block_gram(GramArgs a, int mh, int eb
   for (int t = 0; t < MAXE; t++) {
     int e = ebase + et + t * GT;
     if (ei[t] < 0) continue;
-    double q[4] = {Real<HI>::to_double(hacc_a[t].re), Real<HI>::to_double(hacc_a[t].im),
-                   Real<HI>::to_double(hacc_m[t].re), Real<HI>::to_double(hacc_m[t].im)};
+    double q[4] = {0.0, 0.0, 0.0, 0.0};
+    if constexpr (!ALLLO) {
+      q[0] = Real<HI>::to_double(hacc_a[t].re); q[1] = Real<HI>::to_double(hacc_a[t].im);
+      q[2] = Real<HI>::to_double(hacc_m[t].re); q[3] = Real<HI>::to_double(hacc_m[t].im);
+    }
     if constexpr (!ALLHI) {
       q[0] += (double) acc_a[t].re; q[1] += (double) acc_a[t].im;
       q[2] += (double) acc_m[t].re; q[3] += (double) acc_m[t].im;
@@ -1160,15 +1170,12 @@ extern "C" int mxk_block_gram(int n, int m, int K, const double* ph, mxk_kappa k
     size_t sm = gram_split_smem();
     allow_smem(k_block_gram_split);
     k_block_gram_split<<<dim3(a.chunks, K, nb > 1 ? 2 : 1), GS_T, sm, st>>>(a);
-  } else if (hi_dd) {
-    allow_smem(k_block_gram<dd, false>);
-    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<dd, false><<<g, GT, smem, st>>>(a, mh, eb);
-  } else if (all128) {
-    allow_smem(k_block_gram<double, true>);
-    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, true><<<g, GT, smem, st>>>(a, mh, eb);
   } else {
-    allow_smem(k_block_gram<double, false>);
-    for (int eb = 0; eb < nent; eb += 5 * GT) k_block_gram<double, false><<<g, GT, smem, st>>>(a, mh, eb);
+    auto kern = hi_dd ? k_block_gram<dd, FIRST_HIGH>
+              : all128 ? k_block_gram<double, ALL_HIGH>
+              : mh > 0 ? k_block_gram<double, FIRST_HIGH> : k_block_gram<double, NONE_HIGH>;
+    allow_smem(kern);
+    for (int eb = 0; eb < nent; eb += 5 * GT) kern<<<g, GT, smem, st>>>(a, mh, eb);
   }
   MX_CHECK_LAUNCH();
   size_t work = (size_t) nent * K;
