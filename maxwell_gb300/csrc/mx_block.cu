@@ -286,7 +286,7 @@ template <> struct HiStore<double> { using T = double2; };
 // entry of their own share the sites.  11 c128 vectors, 120^2, 5 k-points:
 // 0.51 -> 0.26 ms.  Of c64 blocks three CTAs fit an SM, which counts where the
 // k-points make more CTAs than two each hold (64^2 x 32, 48 k-points, through
-// gram_edge2d_gpu: 0.87 ms with two, 0.69 with three).
+// gram_edge2d_gpu: 0.81 ms with two, 0.69 with three).
 enum { NONE_HIGH, FIRST_HIGH, ALL_HIGH };
 template <typename HI, int HIGH>
 __global__ void __launch_bounds__(GT, HIGH == NONE_HIGH ? 3 : 2) k_block_gram(GramArgs a, int mh, int ebase) {

@@ -56,6 +56,8 @@ typedef struct {
   double d;
   float hi, lo;
 } mxk_scalar;
+/* out[i] = beta[i] / 6, device arrays */
+int mxk_mass_scalars(size_t count, const double *beta, mxk_scalar *out, mx_stream s);
 /* y = cy*(yin ? yin : y) + alpha*A x + beta*M x, with a beta of its own per
  * (k, vector) where mm_kv (K*m device scalars beta / 6) is not NULL; yin
  * (precision prec_y) may be NULL; cy = 0 reads neither */

@@ -2050,6 +2050,20 @@ extern "C" int mxk_afw_factors(int n, const float* kappa_f, double alpha, double
   return 0;
 }
 
+static __global__ void k_mass_scalars(size_t count, const double* __restrict__ beta, Sc* __restrict__ out) {
+  const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  const double d = beta[i] / 6.0;
+  const float hi = (float) d;
+  out[i] = Sc{d, hi, (float) (d - (double) hi)};
+}
+
+extern "C" int mxk_mass_scalars(size_t count, const double* beta, mxk_scalar* out, mx_stream s) {
+  k_mass_scalars<<<nblocks(count, 256), 256, 0, (cudaStream_t) s>>>(count, beta, (Sc*) out);
+  MX_CHECK_LAUNCH();
+  return 0;
+}
+
 extern "C" int mxk_edge_apply(int n, int m, int K, const double* ph, mxk_kappa kap, double alpha,
                               double beta, const mxk_scalar* mm_kv, double cy, int px, const void* x,
                               int py, const void* yin, void* y, mx_stream s) {

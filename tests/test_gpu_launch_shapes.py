@@ -480,3 +480,23 @@ def test_colour_smoother_batch_shape(n, m, K):
             runs.append(time.perf_counter() - t)
         times.append(sorted(runs[1:])[2])
     assert times[0] < 2.0 * times[1]
+
+
+@pytest.mark.parametrize("K, m", [(32, 32), (41, 25), (3000, 1)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+def test_shifts_of_many_pairs(oracle, K, m, prec):
+    """The operator with a shift per (k-point, vector): the most pairs whose
+    shifts are converted on the host (1024), one more and many."""
+    n = 6
+    rng = np.random.default_rng(K)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(-3.0, 3.0, (K, 2)))
+    g = mx.Grid(n, K, kap, fac)
+    x, y, shift = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n), rng.uniform(-60.0, 0.0, (K, m))
+    ex, ey = mx.Edge(g, m, prec, x), mx.Edge(g, m, prec, y)
+    mx.check(mx.lib().addeval_shifted_edge2d_gpu(1.3, mx._ptr(shift), ex.h, ey.h))
+    got = ey.get()
+    for k in {0, K // 3, K - 1}:
+        for v in range(m):
+            want = oracle.addeval_edge(n, kap, *fac[k], 1.3, shift[k, v], x[k, v], y[k, v])
+            assert rel(got[k, v], want) < TOL[prec]
