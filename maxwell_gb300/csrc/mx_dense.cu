@@ -631,7 +631,12 @@ size_t jacobi_smem(int N) {
 
 extern "C" int mxk_hpd_inverse(int N, int K, double* a, int* info, mx_stream s) {
   const size_t smem = sweep_smem(N);
-  if (smem <= 208 * 1024) {   // orders up to 160
+  // The sweep for orders up to 160, but not where small matrices outnumber the
+  // SMs: a warp takes a column of theirs, and the FP64 unit, which all of an
+  // SM's matrices share, works for idle lanes (Gauss-Jordan against sweep, us:
+  // 300 matrices of order 16 51 / 64, of 32 164 / 171, of 48 445 / 446; 3000 of
+  // 8 88 / 138, of 32 1300 / 1430; 64 of 32 125 / 102).
+  if (smem <= 208 * 1024 && !(N <= 32 && K > 152)) {
     allow_smem(k_hpd_inverse_sweep);
     k_hpd_inverse_sweep<<<K, SWT, smem, (cudaStream_t) s>>>(N, a, info);
   } else {

@@ -500,3 +500,24 @@ def test_shifts_of_many_pairs(oracle, K, m, prec):
         for v in range(m):
             want = oracle.addeval_edge(n, kap, *fac[k], 1.3, shift[k, v], x[k, v], y[k, v])
             assert rel(got[k, v], want) < TOL[prec]
+
+
+@pytest.mark.parametrize("n", [1, 8, 31, 32, 33])
+def test_hermitian_inverses_of_many(n):
+    """Inverses of more small matrices than there are SMs (orders up to 32
+    take a form of their own) and of an order beyond; one of them indefinite.
+    Bound as in test_hermitian_inverse_orders."""
+    rng = np.random.default_rng(n)
+    K = 200
+    A, info = mx.Matrix(n, K), np.zeros(K, np.int32)
+    q = [np.linalg.qr(cv(rng, n, n))[0] for _ in range(K)]
+    a = np.array([(u * np.linspace(1.0, 10.0, n)) @ u.conj().T for u in q])
+    a = (a + np.conj(np.transpose(a, (0, 2, 1)))) / 2
+    A.put(a)
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    assert not info.any()
+    assert rel(A.get(), np.linalg.inv(a)) < 100 * n * 2.2e-16
+    a[7] -= 20.0 * np.eye(n)
+    A.put(a)
+    mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
+    assert info[7] != 0 and info.astype(bool).sum() == 1
