@@ -311,15 +311,20 @@ __device__ void jacobi_sweeps(int N, int ld, Cx<T>* A, Cx<T>* Zm, double* shd, i
 }
 
 // eigenvalues (the diagonal of A) ascending into w, the columns of Zm in the
-// same order; A is overwritten
+// same order; A is overwritten.  An eigenvalue that is NaN keeps its place and
+// the numbers ascend around it: the ranks are a permutation in any case.
 __device__ void sort_eigen(int N, int ld, Cx<double>* A, Cx<double>* Zm, double* w, int* rank) {
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const double wi = AM(A, i, i).re;
-    int r = 0;
+    int r = 0, nans = 0;
     for (int j = 0; j < N; j++) {
       const double wj = AM(A, j, j).re;
       r += wj < wi || (wj == wi && j < i);
+      nans += wj != wj;
     }
+    if (wi != wi) r = i;
+    else if (nans)
+      for (int j = 0; j < N && j <= r; j++) r += AM(A, j, j).re != AM(A, j, j).re;
     rank[i] = r;
     w[r] = wi;
   }

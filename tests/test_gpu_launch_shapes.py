@@ -521,3 +521,28 @@ def test_hermitian_inverses_of_many(n):
     A.put(a)
     mx.check(mx.lib().potrf_matrix_gpu(A.h, mx._ptr(info)))
     assert info[7] != 0 and info.astype(bool).sum() == 1
+
+
+@pytest.mark.parametrize("n", [4, 33, 70])
+def test_eigenvalues_with_nan(n):
+    """A NaN on the diagonal stays there and the other eigenvalues ascend
+    around it, each with its eigenvector; a pencil that turns NaN as a whole
+    reports that or NaN eigenvalues."""
+    K = 2
+    d = np.arange(1.0, n + 1.0)[::-1]
+    a = np.array([np.diag(d), np.diag(d)]).astype(complex)
+    a[1, 2, 2] = np.nan
+    A, info, lam = mx.Matrix(n, K), np.zeros(K, np.int32), np.zeros((K, n))
+    A.put(a)
+    mx.check(mx.lib().syev_matrix_gpu(A.h, mx._ptr(lam), mx._ptr(info)))
+    assert np.array_equal(lam[0], np.sort(d))
+    assert np.array_equal(np.delete(lam[1], 2), np.sort(np.delete(d, 2))) and np.isnan(lam[1, 2])
+    z = np.abs(A.get())
+    assert np.array_equal(z[0], np.eye(n)[:, ::-1])
+    assert np.array_equal(np.sort(z[1].argmax(0)), np.arange(n)) and np.array_equal(z[1].sum(0), np.ones(n))
+    A.put(a)
+    B = mx.Matrix(n, K)
+    B.put(np.array([np.eye(n)] * K))
+    mx.check(mx.lib().sygv_matrix_gpu(A.h, B.h, mx._ptr(lam), mx._ptr(info)))
+    assert info[0] == 0 and np.abs(lam[0] - np.sort(d)).max() < 1e-12 * n
+    assert info[1] != 0 or np.isnan(lam[1]).all()
