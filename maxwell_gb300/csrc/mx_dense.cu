@@ -683,10 +683,8 @@ extern "C" int mxk_rayleigh_ritz(int ns, int m, int K, const double* ga, const d
                                  double* work, mx_stream s) {
   size_t smem = jacobi_smem(ns) + sizeof(int) * (2 * ns + 4) + sizeof(double) * (3 * ns + 2);
   int in_smem = ns <= 48;
-  if (in_smem) {
-    smem += 16 + sizeof(double) * 2 * (size_t) ritz_ld(ns) * ns * 5;
-    allow_smem(k_rayleigh_ritz);
-  }
+  if (in_smem) smem += 16 + sizeof(double) * 2 * (size_t) ritz_ld(ns) * ns * 5;
+  if (smem > 48 * 1024) allow_smem(k_rayleigh_ritz);   // (the rotation data alone from order 939 on)
   int threads = in_smem ? 512 : 1024;
   k_rayleigh_ritz<<<K, threads, smem, (cudaStream_t) s>>>(ns, m, ga, gm, sel, drop, theta_min, coef, theta, info,
                                                          work, in_smem);

@@ -546,3 +546,15 @@ def test_eigenvalues_with_nan(n):
     mx.check(mx.lib().sygv_matrix_gpu(A.h, B.h, mx._ptr(lam), mx._ptr(info)))
     assert info[0] == 0 and np.abs(lam[0] - np.sort(d)).max() < 1e-12 * n
     assert info[1] != 0 or np.isnan(lam[1]).all()
+
+
+def test_pencils_of_large_order():
+    """Generalised eigenvalues of orders whose rotation data alone takes more
+    than 48 KB of shared memory (diagonal matrices: nothing to rotate)."""
+    n = 940
+    d = np.linspace(1.0, 2.0, n)
+    A, B, info, lam = mx.Matrix(n, 1), mx.Matrix(n, 1), np.zeros(1, np.int32), np.zeros(n)
+    A.put(np.diag(d))
+    B.put(np.eye(n))
+    mx.check(mx.lib().sygv_matrix_gpu(A.h, B.h, mx._ptr(lam), mx._ptr(info)))
+    assert info[0] == 0 and np.abs(lam - d).max() < 1e-12
