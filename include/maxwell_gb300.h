@@ -417,12 +417,16 @@ int mxg_kernel_bench(int n, int K, int m, int reps, mxg_kbench_row *rows, int ma
  * width (positions) and band height (pairs of rows) per CTA, and from which
  * batch the node V-cycle's residual + restriction walks strips of coarse
  * rows (coarse nodes x vectors x k-points >= 2^restrict_strip_log2) instead
- * of taking a thread per coarse node. */
+ * of taking a thread per coarse node.  They apply to the launches that
+ * follow; a solver replays, level by level, the launches of its first solve.
+ * A node_strip that fits a level takes its sweeps from the band kernels too,
+ * which a V-cycle of c64 levels otherwise runs (strip 0: bands and one launch
+ * for the coarse levels where they serve, the in-place row kernels elsewhere). */
 typedef struct {
   int gram_waves;        /* 1 .. 64 */
   int combine_ctas;      /* 1 .. 16 */
   int residual_sites;    /* 1 .. 1024 */
-  int node_strip;        /* 0 (the in-place row kernels), 64 or 128 */
+  int node_strip;        /* 0 (no tiled sweep), 64 or 128 */
   int node_band;         /* 1 .. 256 */
   int restrict_strip_log2; /* 0 .. 62 (0: always strips, 62: never) */
 } mxg_tuning;

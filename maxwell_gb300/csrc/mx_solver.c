@@ -117,6 +117,7 @@ struct mxg_solver {
   int all_columns;                    /* Ritz basis with every search column (refinement) */
   int device;                         /* the CUDA device the solver lives on */
   int planar[MAXL];                   /* the lifting of level l runs on planar node vectors */
+  int graph_planar[MAXL];             /* the same in its graph */
 };
 
 #define L_(x) do { int e_ = (x); s->launches++; if (e_) return e_; } while (0)
@@ -132,8 +133,6 @@ static mxk_kappa kap(const mxg_solver *s, int l)
 
 static size_t elen(const mxg_solver *s, int l) { return (size_t) s->K * 2 * s->n[l] * s->n[l] * s->m; }
 static size_t nlen(const mxg_solver *s, int l) { return (size_t) s->K * s->n[l] * s->n[l] * s->m; }
-
-static int planar_level(const mxg_solver *s, int l);
 
 static int dalloc(void **p, size_t bytes)
 {
@@ -284,7 +283,6 @@ mxg_solver *mxg_solver_new(const mxg_solve_opts *o, const double *kappa_fine)
     goto fail;
   s->E0 = s->E;
   s->P0 = s->P;
-  for(l = 1; l <= o->L; l++) s->planar[l] = planar_level(s, l);
   s->gscratch_bytes = (size_t) K * 256 * (ns * (ns + 1) / 2) * 4 * sizeof(double);
   if(s->gscratch_bytes > ((size_t) 1 << 30)) s->gscratch_bytes = (size_t) 1 << 30;
   if(dalloc((void **) &s->gscratch, s->gscratch_bytes)) goto fail;
@@ -483,8 +481,7 @@ static int fused_level(const mxg_solver *s, int top)
 
 /* The lifting of level l runs on planar vectors when every level of its node
  * V-cycle has a kernel of that form: the bands of the fine levels, one launch
- * for the rest (the opt-in tiled sweep keeps its own layout).  Decided when
- * the solver is made: its CUDA graphs hold the choice. */
+ * for the rest (the opt-in tiled sweep keeps its own layout). */
 static int planar_level(const mxg_solver *s, int l)
 {
   int lc, q;
@@ -593,12 +590,16 @@ static int lift_body(mxg_solver *s, int l)
   return 0;
 }
 
+/* The layout of the node vectors follows the tuning at the time of the
+ * launches; a level's graph keeps the one it was captured with. */
 static int lift(mxg_solver *s, int l, int py, void *y)
 {
-  int n = s->n[l];
+  int n = s->n[l], replay = s->graphs && !s->prof && s->glift[l];
   if(s->o.gradient_steps <= 0) return 0;
+  s->planar[l] = replay ? s->graph_planar[l] : l > 0 && planar_level(s, l);
   L_(mxk_adjgradient(n, s->m, s->K, s->ph, 1.0, 1, 0.0, s->planar[l], py, y, s->pg, s->bg[l], s->st));
   TRY(run_graphed(s, l, &s->glift[l], &s->glift_n[l], lift_body));
+  if(!replay && !s->prof && s->glift[l]) s->graph_planar[l] = s->planar[l];
   L_(mxk_gradient(n, s->m, s->K, s->ph, -1.0, s->planar[l], s->pg, s->xg[l], py, y, s->st));
   return 0;
 }

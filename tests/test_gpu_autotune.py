@@ -41,3 +41,35 @@ def test_autotune_choice_and_solve(golden):
             assert res.max() <= float(g["tol"])
     finally:
         mx.set_tuning(**default)
+
+
+def test_tuning_before_the_first_solve():
+    """A node sweep chosen after a solver is made and before its first solve
+    takes effect (the launches of that solve are those of a solver made under
+    the choice), and stays with the solver's graphs afterwards."""
+    default = mx.get_tuning()
+    n0, L, m = 8, 4, 4
+    kap = np.full((n0 << L) ** 2, 0.5)
+    fac = np.exp(1j * np.array([[0.9, 1.7]]))
+
+    def solver():
+        return mx.Solver(kap, n0=n0, L=L, ieigs=2, m=m, method=1, precision=1, max_nested=3, max_steps=2, wave=1,
+                         relative=1, tol=1e-30)
+
+    def launches(s, **tuning):
+        mx.set_tuning(**{**default, **tuning})
+        s.solve(fac)
+        return s.stats()[1]
+
+    try:
+        mx.set_tuning(**default)
+        early = solver()
+        bands = launches(solver())
+        tiled = launches(early, node_strip=64)
+        mx.set_tuning(**{**default, "node_strip": 64})
+        late = solver()
+        assert launches(solver(), node_strip=64) == tiled != bands
+        assert launches(late, node_strip=0) == bands
+        assert launches(early, node_strip=0) == tiled
+    finally:
+        mx.set_tuning(**default)
