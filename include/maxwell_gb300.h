@@ -434,7 +434,8 @@ int mxg_get_tuning(mxg_tuning *t);
 int mxg_set_tuning(const mxg_tuning *t);
 /* Times each shape's candidates (`reps` calls after one untimed call, CUDA
  * events) on synthetic blocks of n x n cells, K k-points and block m <= 16,
- * one tunable after the other, keeps the fastest and returns the choice.
+ * one tunable after the other (the node sweep as both sides of a V-cycle's
+ * level), keeps the fastest and returns the choice.
  * The block kernels' shapes change launch geometry only (results the same
  * up to the order of floating-point sums); the node sweep's strip width
  * also moves where its truncated prefix sums start, at the 8^-9 level. */

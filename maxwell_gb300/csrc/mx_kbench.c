@@ -250,26 +250,35 @@ static int run(int n, int K, int m, int reps, mxg_kbench_row *rows, int maxrows,
     tune->restrict_strip_log2 = mxk_node_rr_get_strips();
     mxk_node_gs_oop_get_shape(&tune->node_strip, &tune->node_band);
     {
-      /* the node sweep: the in-place row kernels (strip 0) against the
-       * tiled out-of-place sweep with each strip x band (two sweeps, so
-       * that both leave the result where the in-place pair does) */
+      /* the node sweep, as both sides of a V-cycle's level with two sweeps
+       * each: strip 0 (the band kernels where they serve, else the in-place
+       * row kernels) against the tiled out-of-place sweep with each strip x
+       * band */
       static const int strips[] = {0, 64, 128}, bands[] = {4, 8, 16, 32, 64};
+      const int nc = n / 2;
       int si, bi, bs = 0, bb = tune->node_band;
       best = 1e30f;
       for(si = 0; si < 3; si++)
         for(bi = 0; bi < (si ? 5 : 1); bi++) {
-          int ok;
+          int tiled;
           TRY(mxk_node_gs_oop_shape(strips[si], si ? bands[bi] : bb));
-          ok = mxk_node_gs_oop_ok(n, m, MX_C64);
-          if(si && !ok) continue;
-#define SWEEP2()                                                                             \
-          (ok ? (mxk_node_gs_oop(n, m, K, ph, 1.0, 0, MX_C64, nb, nx, nd, st)                \
-                 || mxk_node_gs_oop(n, m, K, ph, 1.0, 0, MX_C64, nb, nd, nx, st))            \
-              : (mxk_node_gs(n, m, K, ph, 1.0, 0, MX_C64, nb, nx, st)                        \
-                 || mxk_node_gs(n, m, K, ph, 1.0, 0, MX_C64, nb, nx, st)))
-          TRY(SWEEP2());
+          tiled = mxk_node_gs_oop_ok(n, m, MX_C64);
+          if(si && !tiled) continue;
+#define SWEEP2(DIR)                                                                          \
+          (tiled ? (mxk_node_gs_oop(n, m, K, ph, 1.0, DIR, MX_C64, nb, nx, nd, st)           \
+                    || mxk_node_gs_oop(n, m, K, ph, 1.0, DIR, MX_C64, nb, nd, nx, st))       \
+                 : (mxk_node_gs(n, m, K, ph, 1.0, DIR, MX_C64, nb, nx, st)                   \
+                    || mxk_node_gs(n, m, K, ph, 1.0, DIR, MX_C64, nb, nx, st)))
+#define LEVEL()                                                                              \
+          (!tiled && mxk_node_band_ok(n, m, 2, MX_C64)                                       \
+           ? (mxk_node_band_pre(n, m, K, 2, ph, nb, nx, nd, nbc, st)                         \
+              || mxk_node_band_post(n, m, K, 2, ph, nb, nd, nbc, nx, st))                    \
+           : (SWEEP2(0) || mxk_node_residual_restrict(nc, m, K, ph, 1.0, MX_C64, nx, nb, nbc, st) \
+              || mxk_node_prolong(nc, m, K, ph, 1.0, MX_C64, nbc, nx, st) || SWEEP2(1)))
+          TRY(LEVEL());
           TRY((int) cudaEventRecord(e0, st));
-          for(it = 0; it < reps; it++) TRY(SWEEP2());
+          for(it = 0; it < reps; it++) TRY(LEVEL());
+#undef LEVEL
 #undef SWEEP2
           TRY((int) cudaEventRecord(e1, st));
           TRY((int) cudaEventSynchronize(e1));

@@ -73,3 +73,36 @@ def test_tuning_before_the_first_solve():
         assert launches(early, node_strip=0) == tiled
     finally:
         mx.set_tuning(**default)
+
+
+@pytest.mark.parametrize("L, K", [(5, 4), (6, 2)])
+def test_autotune_does_not_slow_the_solver(L, K):
+    """A solver under the chosen shapes is no slower than under the default
+    ones (with a tenth for the timing; a tiled node sweep chosen against the
+    row kernels, which these levels no longer run, cost it 28 to 32 %)."""
+    import time
+    default = mx.get_tuning()
+    n0, m = 8, 16
+    n = n0 << L
+    i = np.arange(n) / n
+    X, Y = np.meshgrid(i, i)
+    kap = np.where((X - 0.5) ** 2 + (Y - 0.5) ** 2 <= 0.09, 1.0 / 12.0, 1.0).reshape(-1)
+    t = np.linspace(0.3, 2.5, K)
+
+    def seconds():
+        s = mx.Solver(kap, n0=n0, L=L, ieigs=12, m=m, method=1, precision=1, max_nested=20, nested_tol=1e-2,
+                      max_steps=40, wave=K, relative=1, tol=1e-7)
+        times = []
+        for _ in range(4):
+            t0 = time.perf_counter()
+            s.solve(np.exp(1j * np.stack([t, 0.4 * t], 1)))
+            times.append(time.perf_counter() - t0)
+        return min(times[1:])
+
+    try:
+        mx.set_tuning(**default)
+        before = seconds()
+        mx.autotune(n, K, m, 3)
+        assert seconds() < 1.1 * before
+    finally:
+        mx.set_tuning(**default)
