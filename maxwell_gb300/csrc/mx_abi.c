@@ -656,8 +656,9 @@ int adjgradient_node2d_gpu(mxg_field alpha, const edge2d_gpu *x, node2d_gpu *y)
 
 /* The level from which vcycle_node2d_gpu runs in one launch (0: none): a
  * coarse inverse, grids that halve from level to level with the same Bloch
- * factors, vectors of one shape and precision. */
-static int fused_level_n(int L, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x)
+ * factors, vectors of one shape and precision (d too, although the launch does
+ * not use it: another precision is an error). */
+static int fused_level_n(int L, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
 {
   const grid2d_gpu *g0 = x[0]->gr;
   int c, l;
@@ -667,7 +668,7 @@ static int fused_level_n(int L, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu
     const grid2d_gpu *g = x[l]->gr;
     if(g->n != g0->n << l || g->K != g0->K || memcmp(g->h_ph, g0->h_ph, sizeof(double) * 4 * g0->K)
        || x[l]->m != x[0]->m || x[l]->prec != x[0]->prec || b[l]->m != x[0]->m || b[l]->prec != x[0]->prec
-       || b[l]->gr->n != g->n || b[l]->gr->K != g->K)
+       || b[l]->gr->n != g->n || b[l]->gr->K != g->K || (l > 0 && d && d[l] && d[l]->prec != x[0]->prec))
       return 0;
   }
   return c;
@@ -728,7 +729,7 @@ static int planar_cycle(int L, int lc, int nu, const matrix_gpu *Ac, node2d_gpu 
 
 int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x, node2d_gpu **d)
 {
-  int l, i, lc = fused_level_n(L, Ac, b, x);
+  int l, i, lc = fused_level_n(L, Ac, b, x, d);
   if(planar_cycle_ok(L, lc, nu, b, x, d)) return planar_cycle(L, lc, nu, Ac, b, x, d);
   if(!mxk_node_vcycle_pays(x[L]->gr->K * x[L]->m, x[L]->prec)) lc = 0;
   for(l = L; l > lc; l--) {

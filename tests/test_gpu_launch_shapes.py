@@ -558,3 +558,18 @@ def test_pencils_of_large_order():
     B.put(np.eye(n))
     mx.check(mx.lib().sygv_matrix_gpu(A.h, B.h, mx._ptr(lam), mx._ptr(info)))
     assert info[0] == 0 and np.abs(lam - d).max() < 1e-12
+
+
+@pytest.mark.parametrize("level", [1, 2])
+def test_node_vcycle_refuses_other_precisions(level):
+    """d of another precision than b and x is refused on every level, those
+    that run in one launch among them."""
+    n0, L = 8, 2
+    b, x, d, A, arr = node_levels(n0, L, 1, 2, mx.C128, FACTORS[:1])
+    b[L].put(np.zeros(b[L].shape))
+    x[L].put(np.zeros(x[L].shape))
+    other = mx.Node(d[level].g, 2, mx.C64)
+    arr[2][level] = other.h
+    assert mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr) == -1
+    arr[2][level] = d[level].h
+    assert mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr) == 0
