@@ -975,6 +975,8 @@ static int cold_start(mxg_solver *s, int K_active)
       if(s->h_info[k]) return MXG_ECONV;
   }
   if(s->timing) fprintf(stderr, "  coarse eigenproblem %.3f s\n", now_s() - t0);
+  if(s->L == 0)   /* the coarse grid is the finest: its eigenvectors need their residuals only */
+    return iterate(s, 0, s->o.max_steps, K_active);
   for(l = 1; l <= s->L; l++) {
     L_(mxk_zero(s->pe, s->En, elen(s, l), s->st));
     L_(mxk_edge_prolong(s->n[l - 1], m, K, s->ph, 1.0, s->pe, s->E, s->En, s->st));

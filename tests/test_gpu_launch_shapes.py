@@ -573,3 +573,23 @@ def test_node_vcycle_refuses_other_precisions(level):
     assert mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr) == -1
     arr[2][level] = d[level].h
     assert mx.lib().vcycle_node2d_gpu(L, 2, A.h, *arr) == 0
+
+
+@pytest.mark.parametrize("n0, m", [(4, 5), (8, 12)])
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_solver_without_refinement(oracle, n0, m, precision):
+    """A hierarchy of one grid: the dense eigenpairs with their residuals.
+    Bound: order times rounding unit times the largest eigenvalue (1e3), and a
+    factor."""
+    rng = np.random.default_rng(n0)
+    kap = rng.uniform(0.3, 1.0, n0 * n0)
+    fac = FACTORS[[0, 2]]
+    s = mx.Solver(kap, n0=n0, L=0, ieigs=m - 2, m=m, method=1, precision=precision, max_nested=20, max_steps=20, wave=2,
+                  relative=1, tol=1e-8)
+    lam, steps, res = s.solve(fac)
+    assert res[:, :m - 2].max() <= 1e-8 and not steps.any()
+    for k, f in enumerate(fac):
+        R = np.linalg.inv(np.linalg.cholesky(oracle.dense_edge(n0, kap, *f, 0.0, 1.0)))
+        want = np.linalg.eigvalsh(R @ oracle.dense_edge(n0, kap, *f, 1.0, 0.0) @ R.conj().T)
+        want = want[np.abs(want) > 1e-8]
+        assert np.abs(lam[k] - want[:m]).max() < 1e-9
