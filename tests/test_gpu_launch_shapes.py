@@ -593,3 +593,69 @@ def test_solver_without_refinement(oracle, n0, m, precision):
         want = np.linalg.eigvalsh(R @ oracle.dense_edge(n0, kap, *f, 1.0, 0.0) @ R.conj().T)
         want = want[np.abs(want) > 1e-8]
         assert np.abs(lam[k] - want[:m]).max() < 1e-9
+
+
+@pytest.mark.parametrize("n0, L, K, m, nu", [(10, 4, 4, 32, 2), (8, 5, 4, 32, 2), (8, 6, 2, 20, 2), (8, 6, 2, 20, 1),
+                                             (10, 5, 4, 32, 2), (14, 3, 4, 32, 1)])
+def test_node_vcycle_tall_bands(oracle, n0, L, K, m, nu):
+    """c64 node V-cycles of batches whose bands are higher than the 8 rows
+    that few vectors get: 16 to 46 rows, other heights on the way down than up
+    (512^2: 16 and 18, 256^2: 44 and 46, 320^2: 24 and 28), last bands of 8 to
+    36 rows."""
+    rng = np.random.default_rng(n0 + L)
+    n = n0 << L
+    fac = FACTORS[[0, 2, 1, 0]][:K]
+    b, x, d, A, arr = node_levels(n0, L, K, m, mx.C64, fac)
+    b[L].put(cv(rng, K, m, n * n))
+    x[L].put(cv(rng, K, m, n * n))
+    rhs, start = b[L].get(), x[L].get()
+    mx.check(mx.lib().vcycle_node2d_gpu(L, nu, A.h, *arr))
+    got = x[L].get()
+    for k, v in [(0, 0), (1, m // 2), (K - 1, m - 1)]:
+        want = node_cycle(oracle, n0, L, fac[k], rhs[k, v], start[k, v], nu)
+        assert rel(got[k, v], want) < 1e-4
+
+
+@pytest.mark.parametrize("n, m, K", [(260, 3, 1), (514, 1, 2), (514, 1, 4)])
+@pytest.mark.parametrize("prec", [mx.C128, mx.CDD, mx.C64])
+@pytest.mark.parametrize("direction", [0, 1])
+def test_row_smoother_table_refill(oracle, n, m, K, prec, direction):
+    """The row-order smoother on rows of more columns than its table of
+    matrices holds (256).  In 64 bits the oracle's residuals are differences
+    of curls of size n^2: its rounding is the bound."""
+    rng = np.random.default_rng(n)
+    kap = 1.0 / (1.0 + 11.0 * rng.random(n * n))
+    fac = np.exp(1j * rng.uniform(0.3, 3.0, (K, 2)))
+    g = mx.Grid(n, K, kap, fac)
+    b, x = cv(rng, K, m, 2 * n * n), cv(rng, K, m, 2 * n * n)
+    eb, ex = mx.Edge(g, m, prec, b), mx.Edge(g, m, prec, x)
+    fn = [mx.lib().gsforward_edge2d_gpu, mx.lib().gsbackward_edge2d_gpu][direction]
+    mx.check(fn(mx.fz(1.0), mx.fz(0.8), eb.h, ex.h))
+    got = ex.get()
+    for k in {0, K - 1}:
+        for v in {0, m - 1}:
+            want = oracle.gs_edge(n, kap, *fac[k], 1.0, 0.8, direction, b[k, v], x[k, v])
+            assert rel(got[k, v], want) < (1e-4 if prec == mx.C64 else 8 * n * n * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("n0, negative", [(4, 3), (8, 5)])
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_negative_coarse_kappa(oracle, n0, negative, precision):
+    """A coarsest grid with negative kappa starts from the pencil of the edge
+    matrices (orders 32, in shared memory, and 128): as many negative
+    eigenvalues as cells, here the wanted ones, against the dense pencil.
+    kappa is so small there that A + M stays definite.  Bound: order times
+    rounding unit times the largest eigenvalue (1e3), and a factor."""
+    rng = np.random.default_rng(n0)
+    kap = rng.uniform(0.3, 1.0, n0 * n0)
+    kap[rng.choice(n0 * n0, negative, replace=False)] = -1e-4
+    m = negative - 1
+    s = mx.Solver(kap, n0=n0, L=0, ieigs=m, m=m, method=1, precision=precision, max_nested=20, max_steps=20, wave=2,
+                  relative=1, tol=1e-8)
+    lam, _, res = s.solve(FACTORS[[0, 2]])
+    assert res.max() <= 1e-8
+    for k, f in enumerate(FACTORS[[0, 2]]):
+        R = np.linalg.inv(np.linalg.cholesky(oracle.dense_edge(n0, kap, *f, 0.0, 1.0)))
+        want = np.linalg.eigvalsh(R @ oracle.dense_edge(n0, kap, *f, 1.0, 0.0) @ R.conj().T)
+        assert (want[:negative] < -1e-8).all() and abs(want[negative]) < 1e-8
+        assert np.abs(lam[k] - want[:m]).max() < 1e-9
