@@ -229,10 +229,11 @@ def fp64_residual_check(mx, n, kap, fac, lam, vec) -> float:
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per timed
 # sequence at 32 k-points, scaled from ncu captures at 8 or 4 k-points (the
 # full 32-k workload holds > 30 GB on the device): node smoothing launch
-# (profiles/node_band_512x512_k8_ncu.md, two sweeps and the restriction), AFW
-# sweep (profiles/afw_rowpair_512x512_k4_ncu.md), Gram
+# (profiles/node_band_512x512_k8_ncu.md: of the ten on the finest level in a
+# lifting one starts from zero, four restrict with x given, five prolongate),
+# AFW sweep (profiles/afw_rowpair_512x512_k4_ncu.md), Gram
 # (profiles/block_gram_split_512x512_k4_ncu.md)
-TRAFFIC_32K = {"node_gs": 4 * 843.6e6, "afw": 8 * 2 * 648.1e6, "gram": 8 * 3.501e9}
+TRAFFIC_32K = {"node_gs": 4 * (560.4e6 + 4 * 853.0e6 + 5 * 840.0e6) / 10, "afw": 8 * 2 * 648.1e6, "gram": 8 * 3.501e9}
 
 
 def run_ours(args):

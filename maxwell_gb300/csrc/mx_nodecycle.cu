@@ -343,11 +343,12 @@ __global__ void __launch_bounds__(NCT) k_node_vcycle(int n0, int top, int m, int
 //
 // Traffic per side: x and b read with B + 11 (PRE) or B + 8 rows for B, x
 // written once, against 2 nu + .. passes of the separate kernels (a sweep 4
-// arrays, residual and restriction 2.25).  Bound by issue and the barriers of
-// the phases (53 % of issue slots, 0.84 GB of DRAM traffic per PRE call at
-// 512^2).  8 k-points x 16 vectors, nu = 2: PRE 0.455 ms at 512^2 against 0.69
-// for two sweeps and residual with restriction, 0.115 against 0.25 at 256^2;
-// POST 0.355 against 0.56 for prolongation and two sweeps.
+// arrays, residual and restriction 2.25).  Bound by the barriers of the
+// phases and by issue (54 % of issue slots in PRE, 49 % in POST; 0.85 and 0.84
+// GB of DRAM traffic at 512^2).  8 k-points x 16 vectors, nu = 2: PRE 0.456 ms
+// at 512^2 (0.411 from zero) against 0.69 for two sweeps and residual with
+// restriction, 0.117 from zero against 0.25 at 256^2; POST 0.357 against 0.56
+// for prolongation and two sweeps.
 // ------------------------------------------------------------------
 constexpr int NBT = 512;
 
@@ -778,7 +779,7 @@ extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
 // multiple of its time, while the row kernels it replaces only then begin to
 // fill the GPU.  One launch against theirs, cycles from 16 and 32 to 4 or 8,
 // from 64, 80 and 96 to 8, 10 and 12 and from 32 and 64 to 16, ms:
-// c64    2048 vectors 0.21/0.22 .. 1.60/1.71 (all between 0.80 and 0.97),
+// c64    2048 vectors 0.21/0.22 .. 1.60/1.71 (all between 0.75 and 0.97),
 //        4096 vectors 0.64/0.40 and 0.97/0.70 (16, 32), 1.46/1.43 (64)
 // FP64   1024 vectors 0.53/0.64 .. 7.2/7.6, 2048 vectors 1.78/1.03 and
 //        3.30/2.55 (16, 32), 6.97/7.02 (64)
