@@ -216,7 +216,10 @@ int residual_restriction_node2d_gpu(mxg_field alpha, const node2d_gpu *b, const 
 int gradient_node2d_gpu(mxg_field alpha, const node2d_gpu *x, edge2d_gpu *y);
 int adjgradient_node2d_gpu(mxg_field alpha, const edge2d_gpu *x, node2d_gpu *y);
 /* vcycle_node2d (node2d.c:1352-1389); b[l], x[l], d[l] below level L and
- * d[L] are work space (their contents after the call are not defined) */
+ * d[L] are work space (their contents after the call are not defined).  The
+ * first call on c64 levels of 100 to 512 nodes a side allocates a vector of
+ * x[L]'s size on the device, which stays with x[L] until that is deleted;
+ * where there is no memory for it the call does without */
 int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2d_gpu **x,
                       node2d_gpu **d);
 int densematrix_node2d_gpu(int fixnull, const grid2d_gpu *gr, matrix_gpu *a);

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(GT, HIGH == NONE_HIGH ? 3 : 2) k_block_gram(Gr
   Seam<HI> sh = seam_load<HI>(a.ph, a.K, k, n);
   // a launch accumulates the entries [ebase, ebase + MAXE*GT) of the lower
   // triangle (ns <= 48: one launch; larger blocks take several)
-  // Few entries (blocks of up to 21 columns alone): the threads split into
+  // Few entries (blocks of up to 15 columns alone): the threads split into
   // ngr groups that take every ngr-th site of a tile and add up at the end
   constexpr int MAXE = 5;
   const int ngr = nent < GT ? (GT / nent < TS ? GT / nent : TS) : 1, gr = ngr > 1 ? (int) threadIdx.x / nent : 0;

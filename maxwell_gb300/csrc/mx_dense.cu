@@ -1,9 +1,11 @@
 // Batched small dense complex linear algebra in FP64 (one CTA per k-point).
-// These matrices are small (coarse grids of 2*8*8 = 128 edges, Ritz systems
-// of at most 3m = 48 columns); the Jacobi sweeps of the Ritz step do most of
-// their rotations in FP32 and finish in FP64 (jacobi_mixed).  They replace
-// the reference's LAPACK calls (linalg.c:48-317):
+// These matrices are small (at n0 = 8 the inverses of 64 nodes and of 128
+// edges, the coarse eigenproblem's matrix of 64 cells; Ritz systems of at most
+// 3m = 96 columns); the Jacobi sweeps of the coarse eigenproblem and the Ritz
+// step do most of their rotations in FP32 and finish in FP64 (jacobi_mixed).
+// They replace the reference's LAPACK calls (linalg.c:48-317):
 //   mxk_hpd_inverse    zpotrf + ztrsm pairs of the coarse-grid solves
+//   mxk_coarse_pairs   zhegv of the coarse start, through the cells' matrix
 //   mxk_heev           zheev (cyclic Jacobi with Brent-Luk parallel ordering)
 //   mxk_rayleigh_ritz  zhegv of the Ritz step, as Cholesky-QR of the Gram
 //                      matrix with column dropping followed by Jacobi
