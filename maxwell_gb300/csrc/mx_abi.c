@@ -731,7 +731,7 @@ int vcycle_node2d_gpu(int L, int nu, const matrix_gpu *Ac, node2d_gpu **b, node2
 {
   int l, i, lc = fused_level_n(L, Ac, b, x, d);
   if(planar_cycle_ok(L, lc, nu, b, x, d)) return planar_cycle(L, lc, nu, Ac, b, x, d);
-  if(!mxk_node_vcycle_pays(x[L]->gr->K * x[L]->m, x[L]->prec)) lc = 0;
+  if(lc > 0 && !mxk_node_vcycle_pays(x[lc]->gr->n, x[L]->gr->K * x[L]->m, x[L]->prec)) lc = 0;
   for(l = L; l > lc; l--) {
     const grid2d_gpu *g = x[l]->gr;
     for(i = 0; i < nu; i++)

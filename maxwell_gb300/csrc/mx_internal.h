@@ -110,9 +110,10 @@ int mxk_node_rr_get_strips(void);
  * level, x starting from zero where zero is set.  mxk_node_vcycle_top: the
  * highest level up to `top` that this form takes (0: none);
  * mxk_node_vcycle_pays: whether it is the faster form for a batch of vecs
- * vectors when no level above takes bands */
+ * vectors, of n nodes a side on the highest level, when no level above takes
+ * bands */
 int mxk_node_vcycle_top(int n0, int top, int prec);
-int mxk_node_vcycle_pays(int vecs, int prec);
+int mxk_node_vcycle_pays(int n, int vecs, int prec);
 int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
                     const double *phases, const double *ainv, const void *ainv_c64, int prec,
                     const void *b, void *x, mx_stream s);

@@ -777,18 +777,23 @@ extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
 
 // A CTA per vector: past the batch that the SMs hold at once the launch takes a
 // multiple of its time, while the row kernels it replaces only then begin to
-// fill the GPU.  One launch against theirs, cycles from 16 and 32 to 4 or 8,
-// from 64, 80 and 96 to 8, 10 and 12 and from 32 and 64 to 16, ms:
-// c64    2048 vectors 0.21/0.22 .. 1.60/1.71 (all between 0.75 and 0.97),
-//        4096 vectors 0.64/0.40 and 0.97/0.70 (16, 32), 1.46/1.43 (64)
-// FP64   1024 vectors 0.53/0.64 .. 7.2/7.6, 2048 vectors 1.78/1.03 and
-//        3.30/2.55 (16, 32), 6.97/7.02 (64)
-// cdd    448 vectors 0.32/0.39 .. 2.37/2.45, 768 vectors 0.58/0.40 and
-//        1.06/0.86 (16, 32), 1.99/1.96 (64), 3.40/2.78 (96)
+// fill the GPU.  The limits by the highest level's nodes a side, n; one launch
+// against theirs, ms, cycles from 16 and 32 to 4 nodes, from 64 to 8, and of
+// FP64 and float-float from 80 and 96, whose highest level is 40 and 48:
+// c64    2048 vectors 0.33/0.36, 0.50/0.60, 0.76/1.01;
+//        4096 0.64/0.40, 0.97/0.70, 1.46/1.43
+// FP64   1024 vectors 0.90/0.92, 1.66/1.84, 3.49/4.10;
+//        1280 1.15/0.98, 2.12/2.38, 4.48/5.41, 6.57/7.13, 9.09/9.37;
+//        1536 1.40/0.99, 2.59/2.44, 5.47/5.82, 8.14/8.30, 10.2/9.92
+// cdd    448 vectors 0.55/0.64, 0.80/1.08, 1.08/1.57, 1.71/1.86, 2.37/2.45;
+//        512 0.70/0.65, 1.02/1.08, 1.39/1.59, 2.19/2.16, 2.69/2.50;
+//        640 0.86/0.65, 1.25/1.10, 1.71/1.85
 // (Under a level that takes bands the launch serves every batch: the bands'
 // planar vectors need it, and they gain more than it loses.)
-extern "C" int mxk_node_vcycle_pays(int vecs, int prec) {
-  return vecs <= (prec == MX_C64 ? 2048 : prec == MX_C128 ? 1024 : 448);
+extern "C" int mxk_node_vcycle_pays(int n, int vecs, int prec) {
+  if (prec == MX_C64) return vecs <= 2048;
+  if (prec == MX_C128) return vecs <= (n < 32 ? 1024 : 1280);
+  return vecs <= (n % 32 ? 448 : 512);   // (rows that fill their lanes)
 }
 
 extern "C" int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,

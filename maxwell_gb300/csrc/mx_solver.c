@@ -476,7 +476,8 @@ static int fused_node_cycles(mxg_solver *s, int l, int cycles, int zero, int pla
  * where no band kernel takes the levels above (0: none) */
 static int fused_level(const mxg_solver *s, int top)
 {
-  return mxk_node_vcycle_pays(s->K * s->m, s->pg) ? mxk_node_vcycle_top(s->n0, top, s->pg) : 0;
+  int lc = mxk_node_vcycle_top(s->n0, top, s->pg);
+  return lc > 0 && mxk_node_vcycle_pays(s->n[lc], s->K * s->m, s->pg) ? lc : 0;
 }
 
 /* The lifting of level l runs on planar vectors when every level of its node
