@@ -2147,12 +2147,13 @@ static int L_edge_gs_rowpair(int n, int m, int K, const double* ph, mxk_kappa ka
     // 1.15 (a row per CTA without the table 2.07), 32^2 x 16 at 64 d 0.47 /
     // 0.36, f 0.50 / 0.46, at 32 f 0.28 / 0.33; 130^2 x 16 at 32 d 2.88 / 2.27;
     // 64^2 x 16 at 64 d 1.23 / 1.29, f 1.46 / 1.49, at 128 d 2.95 / 2.25, f
-    // 2.81 / 2.73.
+    // 2.81 / 2.73; 400^2 x 16 at 10 d 5.66 / 5.44; 512^2 x 16 at 8 d 6.43 /
+    // 6.95, 512^2 x 8 at 16 d 8.21 / 7.22, f 9.77 / 9.47.
     const int h = n / 2;
     const size_t rows = (size_t) h * K;
     const bool whole = h < AFW_PARTS || rows >= 3072 || (m < 8 && n <= 128 && rows >= 512) ||
                        (n <= 16 && rows >= 384) || (m < 32 && n <= 32 && rows >= 1024) ||
-                       (std::is_same<R, dd>::value && rows >= 1920 && (n > 64 || m > 16));
+                       (std::is_same<R, dd>::value && rows >= 1920 && n <= 448 && (n > 64 || m > 16));
     const int nseg = whole ? 1 : AFW_PARTS, part = (h + nseg - 1) / nseg;
     const int pairs = (AFW_TAB_BYTES / (int) sizeof(AfwSlot<R>) - 1) / 2;   // first-colour patches of a table
     const int P = std::min({256 / m, part, pairs}), T = std::min(pairs / P, (part + P - 1) / P);
