@@ -359,7 +359,7 @@ def test_node_vcycle_large_batch_costs_its_sweeps(prec, n0, L, K, m):
             t = time.perf_counter()
             f()
             times.append(time.perf_counter() - t)
-        return sorted(times)[2]
+        return min(times)
 
     assert seconds(whole) < 1.5 * seconds(parts)
 
@@ -433,7 +433,7 @@ def test_row_smoother_batch_shape(prec, n):
                 mx.check(lib.gsforward_edge2d_gpu(one, one, b.h, x.h))
             mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))
             runs.append(time.perf_counter() - t)
-        times.append(sorted(runs[1:])[2])
+        times.append(min(runs[1:]))
     assert times[0] < 1.7 * times[1]
 
 
@@ -478,7 +478,7 @@ def test_colour_smoother_batch_shape(n, m, K):
                 mx.check(lib.gscolour_edge2d_gpu(one, one, b.h, x.h, 0))
             mx.check(lib.norm2_edge2d_gpu(x.h, mx._ptr(dot)))
             runs.append(time.perf_counter() - t)
-        times.append(sorted(runs[1:])[2])
+        times.append(min(runs[1:]))
     assert times[0] < 2.0 * times[1]
 
 
