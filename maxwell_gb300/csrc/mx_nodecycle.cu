@@ -780,7 +780,8 @@ extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
 // fill the GPU.  The limits by the highest level's nodes a side, n; one launch
 // against theirs, ms, cycles from 16 and 32 to 4 nodes, from 64 to 8, and of
 // FP64 and float-float from 80 and 96, whose highest level is 40 and 48:
-// c64    2048 vectors 0.33/0.36, 0.50/0.60, 0.76/1.01;
+// c64    2048 vectors 0.33/0.36, 0.50/0.60, 0.76/1.01, from 96 to 12 1.60/1.71;
+//        3072 0.49/0.39, 0.74/0.68, 1.13/1.30, 2.38/2.07;
 //        4096 0.64/0.40, 0.97/0.70, 1.46/1.43
 // FP64   1024 vectors 0.90/0.92, 1.66/1.84, 3.49/4.10;
 //        1280 1.15/0.98, 2.12/2.38, 4.48/5.41, 6.57/7.13, 9.09/9.37;
@@ -791,9 +792,10 @@ extern "C" int mxk_node_vcycle_top(int n0, int top, int prec) {
 // (Under a level that takes bands the launch serves every batch: the bands'
 // planar vectors need it, and they gain more than it loses.)
 extern "C" int mxk_node_vcycle_pays(int n, int vecs, int prec) {
-  if (prec == MX_C64) return vecs <= 2048;
+  // (a multiple of 32 or 64: rows that fill their lanes)
+  if (prec == MX_C64) return vecs <= (n % 64 ? 2048 : 3072);
   if (prec == MX_C128) return vecs <= (n < 32 ? 1024 : 1280);
-  return vecs <= (n % 32 ? 448 : 512);   // (rows that fill their lanes)
+  return vecs <= (n % 32 ? 448 : 512);
 }
 
 extern "C" int mxk_node_vcycle(int n0, int top, int m, int K, int nu, int cycles, int zero, int planar,
